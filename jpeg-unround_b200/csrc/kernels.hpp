@@ -439,6 +439,15 @@ bool make_iteration_map(CUtensorMap& map, const float* planes, const Geometry& g
 cudaError_t launch_iteration(const CUtensorMap& state, const CUtensorMap& tilde, const IterationParams& p, bool tgv,
                              bool coupled, int cell_rows, int cell_columns, cudaStream_t stream);
 
+// The same iteration as a walk (walk.cu), which takes what iteration_takes says: the default. Its
+// map boxes two rows of `count` planes, a state's and behind them those of x~ that its primal step
+// made; `p.next` lies likewise behind p.dual.out.
+// And planes of less than 2^30 samples: offsets within one are 32 bits of bytes.
+inline bool walk_takes(const Geometry& g) { return g.plane < (std::size_t{1} << 30); }
+bool make_walk_map(CUtensorMap& map, const float* planes, const Geometry& g, int count);
+cudaError_t launch_walk(const CUtensorMap& map, const IterationParams& p, bool tgv, bool coupled, int cell_rows,
+                        int cell_columns, cudaStream_t stream);
+
 // Pictures of rounded samples in one sweep per iteration (iteration.cu): the dual step and the
 // next primal step with its sample-by-sample proximal map; maps as make_iteration_map makes them.
 struct SamplesIterationParams {

@@ -20,12 +20,16 @@ std::string describe(cudaError_t error) {
   return std::string(cudaGetErrorName(error)) + ": " + cudaGetErrorString(error);
 }
 
-// UNROUND_B200_KERNELS=fused runs the iterations that keep nothing as one sweep each
-// (iteration.cu: the dual step and the next primal step, one pass over HBM); otherwise every
-// iteration is the dual sweep and the primal kernels apart, which measure faster on B200.
-bool fused_kernels() {
+// How the iterations that keep nothing run: by default as one launch each, the walk of walk.cu
+// (the dual step and the next primal step, one pass over HBM); with UNROUND_B200_KERNELS=split
+// as the dual sweep and the primal kernels apart, with =fused as the sweep of iteration.cu.
+enum class Kernels { split, fused, walk };
+
+Kernels chosen_kernels() {
   const char* value = std::getenv("UNROUND_B200_KERNELS");
-  return value != nullptr && std::strcmp(value, "fused") == 0;
+  if (value != nullptr && std::strcmp(value, "fused") == 0) return Kernels::fused;
+  if (value != nullptr && std::strcmp(value, "split") == 0) return Kernels::split;
+  return Kernels::walk;
 }
 
 // How pictures of rounded samples iterate: 0 two launches (the dual sweep, then the primal
@@ -86,6 +90,7 @@ struct Solver::Impl {
   float* xts[2] = {nullptr, nullptr};
   int xt_id = 0;
   bool fusable = false;
+  bool walks = false;  // fusable, by the walk of walk.cu
   int cell_rows = 1, cell_columns = 1;
   CUtensorMap iteration_state_maps[2];
   CUtensorMap iteration_tilde_maps[2];
@@ -110,8 +115,9 @@ struct Solver::Impl {
   // group after both launches have run eagerly (which sets up their launchers), made again for
   // the other parity.
   cudaGraphExec_t group_exec = nullptr;
-  int group_parity = -1;
+  int group_parity = -1, group_xt = -1;
   bool plain_dual = false, plain_primal = false;  // a dual(false) and a primal(false) have run
+  bool plain_fused = false;                       // a fused() has run
 
   Impl(const Frame& f, cudaStream_t s) : frame(f), stream(s) {}
 
@@ -142,10 +148,12 @@ struct Solver::Impl {
 
   // A state's fields in one allocation, each field's channels one after another, in the order
   // x, p1, p2, w1, w2, r11, r22, r12: the planes of the sweep's TMA box (sweep.cu).
-  Fields fields(bool with_tgv) {
+  // With `tilde`, x~'s planes lie behind them (the walk's box, walk.cu).
+  Fields fields(bool with_tgv, float** tilde = nullptr) {
     const std::size_t n = g.plane * g.channels;
     const int count = with_tgv ? 8 : 3;
-    float* block = allocate<float>(n * count);
+    float* block = allocate<float>(n * (count + (tilde != nullptr ? 1 : 0)));
+    if (tilde != nullptr) *tilde = block != nullptr ? block + n * count : nullptr;
     Fields f;
     if (block == nullptr) return f;
     f.x = block;
@@ -237,18 +245,20 @@ struct Solver::Impl {
       coefficients.push_back(allocate<double>(c.coefficient_count()));
       components.push_back(d);
     }
-    state[0] = fields(with_tgv);
-    state[1] = fields(with_tgv);
-    tilde = fields(with_tgv);
-    xt = allocate<float>(n);
-    xts[0] = xt;
-    xt_id = 0;
     samples_layout = samples != nullptr ? samples_kernels() : 0;
-    fusable = solving && (samples != nullptr ? samples_layout != 0 && samples_iteration_takes(g)
-                                             : fused_kernels() && iteration_takes(g, components.data(),
-                                                                                  static_cast<int>(components.size())));
+    const Kernels kernels = chosen_kernels();
+    const bool whole = solving && samples == nullptr && kernels != Kernels::split &&
+                       iteration_takes(g, components.data(), static_cast<int>(components.size()));
+    walks = whole && kernels == Kernels::walk && walk_takes(g);
+    fusable = samples != nullptr ? solving && samples_layout != 0 && samples_iteration_takes(g)
+                                 : walks || (whole && kernels == Kernels::fused);
+    for (int s = 0; s < 2; ++s) state[s] = fields(with_tgv, walks ? &xts[s] : nullptr);
+    tilde = fields(with_tgv);
+    if (!walks) xts[0] = allocate<float>(n);
+    xt = xts[0];
+    xt_id = 0;
     if (fusable) {
-      xts[1] = allocate<float>(n);
+      if (!walks) xts[1] = allocate<float>(n);
       cell_rows = components.size() > 1 ? components[1].cell_rows : 1;
       cell_columns = components.size() > 1 ? components[1].cell_columns : 1;
     }
@@ -260,10 +270,16 @@ struct Solver::Impl {
               make_sweep_map(state_maps[1], state[1].x, g, planes) &&
               make_sweep_map(tilde_maps[0], xts[0], g, g.channels) &&
               (!fusable || make_sweep_map(tilde_maps[1], xts[1], g, g.channels));
-      fusable = fusable && swept && make_iteration_map(iteration_state_maps[0], state[0].x, g, planes) &&
-                make_iteration_map(iteration_state_maps[1], state[1].x, g, planes) &&
-                make_iteration_map(iteration_tilde_maps[0], xts[0], g, g.channels) &&
-                make_iteration_map(iteration_tilde_maps[1], xts[1], g, g.channels);
+      if (walks) {
+        fusable = swept && make_walk_map(iteration_state_maps[0], state[0].x, g, planes + g.channels) &&
+                  make_walk_map(iteration_state_maps[1], state[1].x, g, planes + g.channels);
+        walks = fusable;
+      } else {
+        fusable = fusable && swept && make_iteration_map(iteration_state_maps[0], state[0].x, g, planes) &&
+                  make_iteration_map(iteration_state_maps[1], state[1].x, g, planes) &&
+                  make_iteration_map(iteration_tilde_maps[0], xts[0], g, g.channels) &&
+                  make_iteration_map(iteration_tilde_maps[1], xts[1], g, g.channels);
+      }
       // The primal step's maps: a channel's x, p1 and p2 planes, `channels` planes apart.
       for (std::size_t c = 0; c < components.size(); ++c) {
         bool made = primal_tma_takes(components[c]);
@@ -495,6 +511,10 @@ struct Solver::Impl {
   // (Cb and Cr) in one launch.
   void primal(bool keep) {
     plain_primal = plain_primal || !keep;
+    if (walks) {  // x~ lies behind the state that it is made from
+      xt_id = current;
+      xt = xts[xt_id];
+    }
     if (samples != nullptr) {
       const Fields& st = state[current];
       SamplesPrimalParams sp;
@@ -582,23 +602,26 @@ struct Solver::Impl {
   // launches depend on the iteration only through the parity of the state, which an even count
   // of iterations leaves as it found it.
   bool group() {
-    if (!plain_dual || !plain_primal || fusable || samples != nullptr || error != cudaSuccess || !group_graphs()) {
-      return false;
-    }
-    if (group_exec == nullptr || group_parity != current) {
+    const bool ready = fusable ? walks && plain_fused : plain_dual && plain_primal;
+    if (!ready || samples != nullptr || error != cudaSuccess || !group_graphs()) return false;
+    if (group_exec == nullptr || group_parity != current || group_xt != xt_id) {
       if (group_exec != nullptr) {
         cudaGraphExecDestroy(group_exec);
         group_exec = nullptr;
       }
-      const int parity = current;
+      const int parity = current, buffer = xt_id;
       cudaGraph_t graph = nullptr;
       if (cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
         cudaGetLastError();
         return false;
       }
       for (std::uint64_t k = 0; k < kGraphIterations; ++k) {
-        dual(false);
-        primal(false);
+        if (fusable) {
+          fused();
+        } else {
+          dual(false);
+          primal(false);
+        }
       }
       const cudaError_t ended = cudaStreamEndCapture(stream, &graph);
       if (error == cudaSuccess) error = ended;
@@ -606,12 +629,14 @@ struct Solver::Impl {
       if (graph != nullptr) cudaGraphDestroy(graph);
       if (error != cudaSuccess) return false;
       group_parity = parity;
+      group_xt = buffer;
     }
     error = cudaGraphLaunch(group_exec, stream);
     return error == cudaSuccess;
   }
 
   void fused() {
+    plain_fused = true;
     if (samples != nullptr && samples_layout == 2) {
       SamplesStep q;
       q.levels = s_levels;
@@ -652,8 +677,9 @@ struct Solver::Impl {
     for (std::size_t c = 0; c < components.size(); ++c) ip.component[c] = components[c];
     ip.next = xts[1 - xt_id];
     if (error == cudaSuccess) {
-      error = launch_iteration(iteration_state_maps[current], iteration_tilde_maps[xt_id], ip, tgv, plan.coupled,
-                               cell_rows, cell_columns, stream);
+      error = walks ? launch_walk(iteration_state_maps[current], ip, tgv, plan.coupled, cell_rows, cell_columns, stream)
+                    : launch_iteration(iteration_state_maps[current], iteration_tilde_maps[xt_id], ip, tgv,
+                                       plan.coupled, cell_rows, cell_columns, stream);
     }
     current = 1 - current;
     xt_id = 1 - xt_id;
@@ -1094,17 +1120,17 @@ bool Solver::run(std::uint64_t first, const Observer& observer, Outcome& out, Fa
   if (!stopped && first < most) m.primal(recorded(first + 1));
   while (!stopped && iteration < most && m.error == cudaSuccess) {
     const std::uint64_t next = iteration + 1;
+    // D_next, P_{next+1}, ..., D_{next+G-1}, P_{next+G} (G = kGraphIterations) as one graph when
+    // none of them keeps anything.
+    if (next + kGraphIterations - 1 < most && none_recorded(next, next + kGraphIterations) && m.group()) {
+      iteration = next + kGraphIterations - 1;
+      continue;
+    }
     // One sweep for D_next and P_{next+1} when neither keeps anything: no record after the
     // dual step, none of the next iterate, and a next iteration to make.
     if (m.fusable && next < most && !recorded(next) && !recorded(next + 1)) {
       m.fused();
       iteration = next;
-      continue;
-    }
-    // D_next, P_{next+1}, ..., D_{next+G-1}, P_{next+G} (G = kGraphIterations) as one graph when
-    // none of them keeps anything.
-    if (next + kGraphIterations - 1 < most && none_recorded(next, next + kGraphIterations) && m.group()) {
-      iteration = next + kGraphIterations - 1;
       continue;
     }
     if (m.error != cudaSuccess) break;
@@ -1276,15 +1302,15 @@ bool Solver::iterate(std::uint64_t iterations, Failure& failure) {
   std::uint64_t n = 0;
   while (n < iterations && m.error == cudaSuccess) {
     const bool last = n + 1 == iterations;
-    if (m.fusable && !last) {
-      m.fused();
-      ++n;
-      continue;
-    }
     // kGraphIterations iterations as one graph while at least one more (the last, which keeps)
     // follows.
     if (iterations - n > kGraphIterations && m.group()) {
       n += kGraphIterations;
+      continue;
+    }
+    if (m.fusable && !last) {
+      m.fused();
+      ++n;
       continue;
     }
     if (m.error != cudaSuccess) break;
