@@ -284,6 +284,22 @@ unround_status unround_b200_strip_exchange_local(unround_b200_strip* const* stri
                                                  const unround_b200_strip_exchange* exchanges,
                                                  uint64_t exchange_count, char* message, size_t message_size);
 
+/* Host memory for a result's arrays (no counterpart in the reference): a binding copies a result
+ * into arrays of its own, and pages fresh from the system cost more than the copies (a 768x512
+ * colour result is 47 MB in 16 arrays).
+ *   _host_block       at least `bytes` bytes, 16-byte aligned, from blocks returned earlier (2 GiB
+ *                     idle at most, shared with the solver's host model) or the heap; null when
+ *                     there are none
+ *   _host_block_free  returns a block (any thread; null is taken)
+ *   _copy_parts       copies `count` arrays, shared out among the host's threads by bytes
+ *   _result_intervals every component's lower ends, upper ends and centres (as
+ *                     unround_result_problem gives them, 0, 1 and 2) into to[3 c], to[3 c + 1] and
+ *                     to[3 c + 2], the blocks shared out among the host's threads */
+void* unround_b200_host_block(uint64_t bytes);
+void unround_b200_host_block_free(void* block);
+void unround_b200_copy_parts(uint64_t count, void* const* to, const void* const* from, const uint64_t* bytes);
+unround_status unround_b200_result_intervals(const unround_result* result, double* const* to);
+
 /* The failure path of the bounded waits (no counterpart in the reference, whose solver has no
  * device): every wait of a kernel on an mbarrier is bounded, and one that runs out sets an error
  * word that the solve reports as UNROUND_ERROR_INTERNAL ("a bounded wait of the sweep ran out")

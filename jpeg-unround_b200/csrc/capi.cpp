@@ -94,6 +94,24 @@ std::int32_t guarded(char* message, std::size_t size, Body&& body) {
   }
 }
 
+// body(first, end), which does not throw, over [0, total) in `parts` ranges of about the same size, each on a thread; a
+// thread that cannot be had leaves its range to the caller's.
+template <typename Body>
+void in_parts(std::size_t total, std::size_t parts, const Body& body) {
+  std::vector<std::thread> workers;
+  std::size_t made = 1;
+  try {
+    workers.reserve(parts);
+    for (; made < parts; ++made) workers.emplace_back(body, total * made / parts, total * (made + 1) / parts);
+  } catch (...) {
+  }
+  body(0, total / parts);
+  if (made < parts) body(total * made / parts, total);
+  for (std::thread& w : workers) w.join();
+}
+
+std::size_t host_threads() { return std::max(1u, std::min(16u, std::thread::hardware_concurrency())); }
+
 bool have_device(urb::Failure& failure) {
   int count = 0;
   cudaError_t error = cudaGetDeviceCount(&count);
@@ -1054,6 +1072,62 @@ const double* unround_result_problem(const unround_result* result, uint64_t comp
   }
   put(count, result->problem_sizes[component]);
   return result->problem[which][component].get();
+}
+
+void* unround_b200_host_block(uint64_t bytes) {
+  try {
+    return urb::reused_block(static_cast<std::size_t>(bytes));
+  } catch (...) {
+    return nullptr;
+  }
+}
+
+void unround_b200_host_block_free(void* block) {
+  try {
+    urb::return_block(block);
+  } catch (...) {  // no memory to note it as idle
+  }
+}
+
+void unround_b200_copy_parts(uint64_t count, void* const* to, const void* const* from, const uint64_t* bytes) {
+  std::size_t total = 0;
+  for (std::uint64_t k = 0; k < count; ++k) total += bytes[k];
+  auto copy = [&](std::size_t first, std::size_t end) {
+    std::size_t at = 0;  // of array k in the arrays one after another
+    for (std::uint64_t k = 0; k < count && at < end; ++k) {
+      const std::size_t a = std::max(first, at), b = std::min(end, at + bytes[k]);
+      if (a < b) std::memcpy(static_cast<char*>(to[k]) + (a - at), static_cast<const char*>(from[k]) + (a - at), b - a);
+      at += bytes[k];
+    }
+  };
+  // A thread a MiB or more (0.1 ms of copying, above a thread's start).
+  in_parts(total, std::min(host_threads(), std::max<std::size_t>(total >> 20, 1)), copy);
+}
+
+unround_status unround_b200_result_intervals(const unround_result* result, double* const* to) {
+  if (result == nullptr || to == nullptr) return UNROUND_ERROR_ARGUMENT;
+  const auto& components = result->frame.components;
+  std::size_t total = 0;
+  for (const urb::Component& c : components) total += c.coefficient_count() / 64;
+  auto fill = [&](std::size_t first, std::size_t end) {
+    std::size_t at = 0;  // of component c's blocks
+    for (std::size_t z = 0; z < components.size() && at < end; ++z) {
+      const urb::Component& c = components[z];
+      const std::size_t blocks = c.coefficient_count() / 64;
+      const std::size_t a = std::max(first, at), b = std::min(end, at + blocks);
+      for (std::size_t block = a; block < b; ++block) {
+        for (int k = 0; k < 64; ++k) {
+          const std::size_t entry = (block - at) * 64 + k;
+          to[3 * z][entry] = c.lower(c.levels[entry], k);
+          to[3 * z + 1][entry] = c.upper(c.levels[entry], k);
+          to[3 * z + 2][entry] = c.centre(c.levels[entry], k);
+        }
+      }
+      at += blocks;
+    }
+  };
+  in_parts(total, std::min(host_threads(), std::max<std::size_t>(total / 512, 1)), fill);
+  return UNROUND_OK;
 }
 
 unround_status unround_result_component(const unround_result* result, uint64_t component, uint64_t* rows,

@@ -1,9 +1,12 @@
 // The cache of pinned blocks behind HostBuffer. Idle blocks are kept up to kIdleLimit bytes in
-// all; a request takes the smallest idle block that holds it and is at most twice its size, or
-// pins a new one (rounded up to 2 MiB). The cache is never destroyed: the blocks outlive static
+// all; a request, rounded up to 2 MiB, takes the smallest idle block that holds it and is at most
+// twice its size, or pins a new one. (Compared with the size not rounded, no block ever matched a
+// request below 1 MiB: each solve of a small picture pinned new ones, 3 ms of a 160x120 picture's
+// 4.6.) The cache is never destroyed: the blocks outlive static
 // destruction, when the CUDA runtime may be gone, and the process's exit returns them.
 #include "host_buffer.hpp"
 
+#include <algorithm>
 #include <cstdlib>
 #include <map>
 #include <mutex>
@@ -26,6 +29,7 @@ struct Cache {
 
   // A pinned block of at least `bytes` (its size into `got`), or null.
   void* take(std::size_t bytes, std::size_t& got) {
+    bytes = (bytes + kGrain - 1) / kGrain * kGrain;
     {
       std::lock_guard<std::mutex> hold(lock);
       auto it = idle.lower_bound(bytes);
@@ -37,7 +41,7 @@ struct Cache {
         return block;
       }
     }
-    got = (bytes + kGrain - 1) / kGrain * kGrain;
+    got = bytes;
     void* block = nullptr;
     if (cudaHostAlloc(&block, got, cudaHostAllocPortable) != cudaSuccess) {
       cudaGetLastError();  // the failure is not the caller's error
@@ -101,7 +105,7 @@ void HostBuffer::release() {
 void HostBuffer::resize(std::size_t count) {
   const std::size_t bytes = count * sizeof(double);
   if (count == size_) return;
-  if (bytes <= bytes_ && bytes * 2 >= bytes_) {
+  if (bytes <= bytes_ && std::max(bytes, kGrain) * 2 >= bytes_) {
     size_ = count;
     return;
   }

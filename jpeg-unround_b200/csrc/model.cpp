@@ -17,14 +17,21 @@ namespace urb {
 namespace {
 
 // The reused blocks: each starts with a header of its size; idle ones are kept up to kKeep bytes
-// in all, a request taking the smallest idle block that holds it and is at most twice its size.
+// in all (the longest idle go first), a request taking the smallest idle block that holds it and
+// is at most twice its size. 2 GiB hold a 12-megapixel colour result's arrays (1.5 GB) beside its
+// model's.
 constexpr std::size_t kHeader = 64;
-constexpr std::size_t kKeep = std::size_t{1} << 30;
+constexpr std::size_t kKeep = std::size_t{2} << 30;
 
 struct Blocks {
+  struct Idle {
+    void* block;
+    std::uint64_t since;
+  };
   std::mutex lock;
-  std::multimap<std::size_t, void*> idle;  // bytes -> block
+  std::multimap<std::size_t, Idle> idle;  // by bytes
   std::size_t idle_bytes = 0;
+  std::uint64_t returned = 0;
 };
 
 Blocks& blocks() {
@@ -40,7 +47,7 @@ void* reused_block(std::size_t bytes) {
     std::lock_guard<std::mutex> hold(b.lock);
     auto it = b.idle.lower_bound(bytes + kHeader);
     if (it != b.idle.end() && it->first <= 2 * (bytes + kHeader)) {
-      void* block = it->second;
+      void* block = it->second.block;
       b.idle_bytes -= it->first;
       b.idle.erase(it);
       return static_cast<char*>(block) + kHeader;
@@ -57,16 +64,26 @@ void return_block(void* at) {
   if (at == nullptr) return;
   void* block = static_cast<char*>(at) - kHeader;
   const std::size_t size = *static_cast<std::size_t*>(block);
+  if (size > kKeep) {
+    std::free(block);
+    return;
+  }
   Blocks& b = blocks();
+  std::vector<void*> gone;
   {
     std::lock_guard<std::mutex> hold(b.lock);
-    if (b.idle_bytes + size <= kKeep) {
-      b.idle.emplace(size, block);
-      b.idle_bytes += size;
-      return;
+    while (b.idle_bytes + size > kKeep) {
+      const auto oldest = std::min_element(b.idle.begin(), b.idle.end(), [](const auto& x, const auto& y) {
+        return x.second.since < y.second.since;
+      });
+      gone.push_back(oldest->second.block);
+      b.idle_bytes -= oldest->first;
+      b.idle.erase(oldest);
     }
+    b.idle.emplace(size, Blocks::Idle{block, b.returned++});
+    b.idle_bytes += size;
   }
-  std::free(block);
+  for (void* other : gone) std::free(other);
 }
 
 namespace {

@@ -240,6 +240,10 @@ def _bind(library: ctypes.CDLL) -> None:
         "unround_b200_measure": (i32, ctypes.POINTER(_Input), handle, u64, u64, ctypes.POINTER(_Timing),
                                  ctypes.POINTER(handle), *text),
         "unround_b200_model": (i32, ctypes.POINTER(_Input), handle, u64, i32, doubles, u64, u64p, *text),
+        "unround_b200_host_block": (handle, u64),
+        "unround_b200_host_block_free": (None, handle),
+        "unround_b200_copy_parts": (None, u64, ctypes.POINTER(handle), ctypes.POINTER(handle), u64p),
+        "unround_b200_result_intervals": (i32, handle, ctypes.POINTER(handle)),
         "unround_b200_solve_batch": (i32, u64, ctypes.POINTER(_Input), ctypes.POINTER(handle), ctypes.POINTER(handle),
                                      ctypes.POINTER(_BatchTiming), *text),
     }
@@ -496,26 +500,88 @@ def _copy(pointer: object, shape: tuple[int, ...], dtype: type = np.float64) -> 
     return out.reshape(shape)
 
 
+# Arrays of at least this size take blocks of the library's (reused: no fresh pages); smaller ones
+# come from the heap that NumPy takes, which keeps such sizes itself.
+_BLOCK_BYTES: Final = 128 << 10
+
+
+class _Block:
+    """A host block of the library's as an array's base; given back when the last array of it goes."""
+
+    __slots__ = ("__array_interface__", "_free", "_pointer")
+
+    def __init__(self, library: ctypes.CDLL, shape: tuple[int, ...]) -> None:
+        self._pointer = None
+        self._free = library.unround_b200_host_block_free
+        pointer = library.unround_b200_host_block(8 * int(np.prod(shape, dtype=np.int64)))
+        if not pointer:
+            raise MemoryError("no host memory for a result's array")
+        self._pointer = pointer
+        self.__array_interface__ = {"shape": shape, "typestr": "<f8", "data": (pointer, False), "version": 3}
+
+    def __del__(self) -> None:
+        if self._pointer:
+            self._free(self._pointer)
+
+
+def _empty(library: ctypes.CDLL, shape: tuple[int, ...]) -> Array:
+    if 8 * int(np.prod(shape, dtype=np.int64)) < _BLOCK_BYTES:
+        return np.empty(shape)
+    return np.asarray(_Block(library, shape))
+
+
+class _Copies:
+    """The copies of a result's arrays, made together by the library on the host's threads."""
+
+    def __init__(self, library: ctypes.CDLL) -> None:
+        self._library = library
+        self._parts: list[tuple[Array, int]] = []
+
+    def of(self, pointer: object, shape: tuple[int, ...]) -> Array:
+        """An array of the shape, filled from the pointer by run()."""
+        out = _empty(self._library, shape)
+        if out.size:
+            if not pointer:
+                raise RuntimeError("the library gave no values where it has some")
+            self._parts.append((out, ctypes.cast(pointer, ctypes.c_void_p).value or 0))  # type: ignore[arg-type]
+        return out
+
+    def run(self) -> None:
+        count = len(self._parts)
+        to = (ctypes.c_void_p * max(count, 1))(*(out.ctypes.data for out, _ in self._parts))
+        source = (ctypes.c_void_p * max(count, 1))(*(pointer for _, pointer in self._parts))
+        sizes = (ctypes.c_uint64 * max(count, 1))(*(out.nbytes for out, _ in self._parts))
+        self._library.unround_b200_copy_parts(count, to, source, sizes)
+
+
 def _decoded(library: ctypes.CDLL, result: ctypes.c_void_p, problems: bool = True) -> Decoded:
     u = [ctypes.c_uint64() for _ in range(4)]
+    copies = _Copies(library)
     pointer = library.unround_result_picture(result, *(ctypes.byref(x) for x in u[:3]))
     rows, columns, depth = (int(x.value) for x in u[:3])
-    picture = _copy(pointer, (rows, columns) if depth == 1 else (rows, columns, depth))
+    picture = copies.of(pointer, (rows, columns) if depth == 1 else (rows, columns, depth))
     pointer = library.unround_result_canvas(result, *(ctypes.byref(x) for x in u[:3]))
     channels, height, width = (int(x.value) for x in u[:3])
-    canvas = _copy(pointer, (channels, height, width))
+    canvas = copies.of(pointer, (channels, height, width))
     count = ctypes.c_uint64()
-    planes = _copy(library.unround_result_planes(result, ctypes.byref(count)), (channels, rows, columns))
-    coefficients, models = [], []
+    planes = copies.of(library.unround_result_planes(result, ctypes.byref(count)), (channels, rows, columns))
+    coefficients, models, intervals = [], [], []
     for index in range(int(library.unround_result_components(result))):
         library.unround_result_component(result, index, *(ctypes.byref(x) for x in u))
         block_rows, block_columns, down, across = (int(x.value) for x in u)
         shape = (block_rows, block_columns, 8, 8)
-        coefficients.append(_copy(library.unround_result_coefficients(result, index, ctypes.byref(count)), shape))
+        coefficients.append(copies.of(library.unround_result_coefficients(result, index, ctypes.byref(count)), shape))
         if problems:
-            arrays = [_copy(library.unround_result_problem(result, index, which, ctypes.byref(count)),
-                            shape if which < 3 else (8, 8)) for which in range(5)]
-            models.append(Problem((down, across), *arrays))
+            ends = [_empty(library, shape) for _ in range(3)]
+            intervals.extend(ends)
+            tables = [_copy(library.unround_result_problem(result, index, which, ctypes.byref(count)), (8, 8))
+                      for which in (3, 4)]
+            models.append(Problem((down, across), *ends, *tables))
+    copies.run()
+    if intervals:
+        pointers = (ctypes.c_void_p * len(intervals))(*(ends.ctypes.data for ends in intervals))
+        if library.unround_b200_result_intervals(result, pointers) != Status.OK:
+            raise RuntimeError("the library gave no values where it has some")
     iterations, stop = ctypes.c_uint64(), ctypes.c_int32()
     solution = None
     if library.unround_result_solver(result, ctypes.byref(iterations), ctypes.byref(stop)):
