@@ -33,10 +33,10 @@
 // by instruction fetch, so that code size counts (the edges' tests are folded into addresses, and
 // what is rarely run is not inlined: 4032x3024 TV 331 -> 261 us). Its rows are there when a chunk
 // begins: of 56 looks at the ring, 55 need no wait. Measured, an iteration as graphs of eight,
-// before (two or three launches) and after: TV grey 160x120 12.6 -> 5.3 us, 512^2 13.3 -> 6.9;
-// TGV grey 512^2 18.4 -> 8.9, 1024^2 25.8 -> 17.5, 4096^2 258 -> 215; TGV 4:2:0 768x512 36.7 ->
-// 20.6, 1919x1083 115 -> 97, 4032x3024 563 -> 550; TV 4:2:0 1919x1083 63.2 -> 58.0, 4032x3024 304
-// -> 261.
+// before (two or three launches) and after: TV grey 160x120 12.6 -> 5.0 us, 512^2 13.3 -> 6.2;
+// TGV grey 512^2 18.4 -> 8.6, 1024^2 25.8 -> 17.5, 4096^2 258 -> 211; TGV 4:2:0 768x512 36.7 ->
+// 19.9, 1919x1083 115 -> 97, 4032x3024 563 -> 536; TV 4:2:0 1919x1083 63.2 -> 46.4, 2048^2 101 (two
+// CTAs an SM, a barrier for each tile) -> 86.
 #include <algorithm>
 #include <atomic>
 #include <type_traits>
@@ -65,6 +65,13 @@ constexpr int walk_threads() {
 constexpr int kSlots = 9;     // of the ring, two rows each: a chunk's and the row below, and the next chunk's
 
 constexpr int round32(int n) { return (n + 31) / 32 * 32; }
+
+// CTAs an SM holds: by shared memory (TGV: 112 KB of three channels, 62 KB of one), else by
+// registers; TV of three channels with two: 8% slower at 2048x2048, 14% at 1919x1083.
+template <bool TGV, int C>
+constexpr int walk_ctas() {
+  return C == 1 ? (TGV ? 3 : 4) : (TGV ? 2 : 3);
+}
 
 // Two neighbouring samples of a row, as the packed binary32 operations take them: each lane of
 // a pair rounded as the operation of single samples.
@@ -296,15 +303,16 @@ __device__ __forceinline__ void prox_rows(float* tile, const Ahead& a, const Wal
   }
 }
 
-// The CTA's barriers. full: a slot's bytes are in; drained: a chunk's rows are read (by the
-// dual step's warps and the side warp), in turns; beside: the left column of a chunk is made, in
-// turns; luma, chroma: a tile of v is whole, and free again.
+// The CTA's barriers. full: a slot's bytes are in; drained: a chunk's rows are read (by the dual
+// step's warps and the left column's), in turns; go: the second part of a chunk may run, in turns
+// (its left column is made, and the proximal maps' warps are done with the tiles it writes);
+// luma, chroma: a tile of v is whole.
 struct WalkBarriers {
   std::uint64_t full[kSlots];
   std::uint64_t drained[2];
-  std::uint64_t beside[2];
-  std::uint64_t luma_full[2], luma_empty[2];
-  std::uint64_t chroma_full[2], chroma_empty[2];
+  std::uint64_t go[2];
+  std::uint64_t luma[2];
+  std::uint64_t chroma[2];
 };
 
 // A barrier of the dual step's warps; whether any of their threads says so.
@@ -316,6 +324,10 @@ __device__ __forceinline__ bool any_of_dual(bool said) {
       : "r"(static_cast<int>(said)), "n"(32 * kDual)
       : "memory");
   return any != 0;
+}
+
+__device__ __forceinline__ void dual_barrier() {
+  asm volatile("barrier.cta.sync 1, %0;" ::"n"(32 * kDual) : "memory");
 }
 
 // Waits for a phase of a barrier that has not come at once, until another warp of the CTA has given
@@ -569,13 +581,7 @@ struct Walk {
         }
         __syncwarp();
         if (lane == 0) barrier_arrive(&bars.drained[k & 1]);
-        // The left column is made, and the tiles of v are free.
-        good = wait_unless(&bars.beside[k & 1], (k >> 1) & 1, failed);
-        if (k >= 2) good = good && wait_unless(&bars.luma_empty[k & 1], ((k >> 1) - 1) & 1, failed);
-        if constexpr (C > 1) {
-          const int band = k / CR;
-          if (band >= 2) good = good && wait_unless(&bars.chroma_empty[band & 1], ((band >> 1) - 1) & 1, failed);
-        }
+        good = wait_unless(&bars.go[k & 1], (k >> 1) & 1, failed);
       }
       if (any_of_dual(!good)) return false;
       {
@@ -593,10 +599,10 @@ struct Walk {
       }
       __syncwarp();
       if (lane == 0) {
-        barrier_arrive(&bars.luma_full[k & 1]);
-        if constexpr (C > 1) barrier_arrive(&bars.chroma_full[k / CR & 1]);
+        barrier_arrive(&bars.luma[k & 1]);
+        if constexpr (C > 1) barrier_arrive(&bars.chroma[k / CR & 1]);
       }
-      any_of_dual(false);  // the exchange is read before the next chunk's is written
+      dual_barrier();  // the exchange is read before the next chunk's is written
     }
     return true;
   }
@@ -659,7 +665,7 @@ struct Walk {
     }
     __syncwarp();
     if (lane == 0) {
-      barrier_arrive(&bars.beside[k & 1]);
+      barrier_arrive(&bars.go[k & 1]);
       barrier_arrive(&bars.drained[k & 1]);
     }
     return true;
@@ -684,32 +690,39 @@ struct Walk {
       if (!__all_sync(kAll, wait_unless(&bars.drained[k & 1], (k >> 1) & 1, failed))) return false;
       issue_to(kSlots + 1 + kDual * (k + 1));
       // The left column of chunk k is read once v of the chunk is made; the next goes beside it.
-      if (k > 0 && !__all_sync(kAll, wait_unless(&bars.luma_full[(k - 1) & 1], ((k - 1) >> 1) & 1, failed))) return false;
+      if (k > 0 && !__all_sync(kAll, wait_unless(&bars.luma[(k - 1) & 1], ((k - 1) >> 1) & 1, failed))) return false;
       if (k + 1 < chunks && !left_column(bars, failed, k + 1, lane)) return false;
     }
     return true;
   }
 
   // ---- The other warps: the proximal map of channel c (its part of the strip), block row by block
-  // row of it, the levels looked up one ahead.
+  // row of it, the levels looked up one ahead. When one of its two tiles is full, the other is free:
+  // the chunks that fill it may go.
   template <int PR, int PC>
   __device__ __forceinline__ bool prox_warp(WalkBarriers& bars, const volatile int* failed, const WalkFactors& F, int c,
                                             int part, int lane) const {
     constexpr int BH = 8 * PR;
     const int j = x0 + 32 * part + lane, pitch = Q.dual.g.pitch;
-    std::uint64_t* const full = c == 0 ? bars.luma_full : bars.chroma_full;
-    std::uint64_t* const empty = c == 0 ? bars.luma_empty : bars.chroma_empty;
+    std::uint64_t* const full = c == 0 ? bars.luma : bars.chroma;
     float* const tile = shared + (c == 0 ? W::LUMA : W::CHROMA + (c - 1) * BH * WIDTH) + 32 * part;
     const int stride = c == 0 ? BH * WIDTH : (C - 1) * BH * WIDTH;
     float* next = Q.next + c * Q.dual.g.plane + static_cast<std::size_t>(i0) * pitch + j;
+    auto let_go = [&](int band) {
+#pragma unroll
+      for (int k = 0; k < PR; ++k) {
+        if (lane == 0) barrier_arrive(&bars.go[(band * PR + k) & 1]);
+      }
+    };
+    let_go(0);
     Ahead ahead = look_ahead<PR, PC>(Q, c, j, i0, lane);
     for (int i = i0, b = 0; i < i1; i += BH, ++b) {
       const Ahead now = ahead;
       if (i + BH < i1) ahead = look_ahead<PR, PC>(Q, c, j, i + BH, lane);
       if (!__all_sync(kAll, wait_unless(&full[b & 1], (b >> 1) & 1, failed))) return false;
+      let_go(b + 1);
       prox_rows<PR, PC, WIDTH>(tile + (b & 1) * stride, now, F, next, pitch, lane, j < Q.dual.g.columns);
       __syncwarp();
-      if (lane == 0) barrier_arrive(&empty[b & 1]);
       next += static_cast<std::size_t>(BH) * pitch;
     }
     return true;
@@ -717,7 +730,7 @@ struct Walk {
 };
 
 template <bool TGV, int C, bool COUPLED, int CR, int CC>
-__global__ void __launch_bounds__(walk_threads<C>(), C == 1 ? 3 : 2)
+__global__ void __launch_bounds__(walk_threads<C>(), walk_ctas<TGV, C>())
     walk_kernel(const __grid_constant__ CUtensorMap map, const __grid_constant__ IterationParams Q) {
   using W = WalkLayout<TGV, C, CR>;
   extern __shared__ __align__(128) float shared[];
@@ -740,11 +753,9 @@ __global__ void __launch_bounds__(walk_threads<C>(), C == 1 ? 3 : 2)
     for (int s = 0; s < kSlots; ++s) barrier_init(&bars.full[s], 1);
     for (int s = 0; s < 2; ++s) {
       barrier_init(&bars.drained[s], kDual + 1);
-      barrier_init(&bars.beside[s], 1);
-      barrier_init(&bars.luma_full[s], kDual);
-      barrier_init(&bars.luma_empty[s], C == 1 ? 2 : 1);
-      barrier_init(&bars.chroma_full[s], kDual * CR);
-      barrier_init(&bars.chroma_empty[s], 2);
+      barrier_init(&bars.go[s], 1 + (C == 1 ? 2 : C));
+      barrier_init(&bars.luma[s], kDual);
+      barrier_init(&bars.chroma[s], kDual * CR);
     }
     failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
