@@ -287,30 +287,6 @@ __global__ void __launch_bounds__(256) dual_stream_kernel(const DualParams P) {
 // for the row DCT, the clip, and the inverse row DCT; a second transpose returns the columns.
 // The interval, the centre and the proximal map of a coefficient are prox.cuh's.
 
-// G's terms at a coefficient in binary64 (cpp/src/model.cpp:384-392): m/2 (c - centre)^2, and
-// the cost of lying beyond the file's own interval.
-__device__ __forceinline__ double value_term(double zeta, int q, int k, bool flat, const Constants64& K) {
-  const double level = static_cast<double>(q);
-  const double step = K.step[k];
-  const double shift = k == 0 ? 1024.0 : 0.0;
-  double centre;
-  if (K.mmse && k != 0) {
-    const double size = (fabs(level) - K.shrink[k]) * step;
-    centre = q == 0 ? 0.0 : (q < 0 ? -size : size);
-  } else {
-    centre = level * step + shift;
-  }
-  const double m = flat ? K.flat_weight[k] : K.weight[k];
-  const double away = zeta - centre;
-  double term = 0.5 * m * (away * away);
-  if (K.costed) {
-    const double own_low = (level - 0.5) * step + shift;
-    const double own_high = (level + 0.5) * step + shift;
-    term = term + K.cost[k] * fmax(fmax(zeta - own_high, own_low - zeta), 0.0);
-  }
-  return term;
-}
-
 // A lane per canvas column: a component block covers 8 CC columns, so a warp takes 32 / (8 CC)
 // blocks side by side (one for CC = 3, its last 8 lanes idle), and walks down kPrimalRows block
 // rows. The CC lanes of a cell's columns sum their columns and exchange the sums (in the
@@ -1265,13 +1241,14 @@ __device__ __forceinline__ double conjugate_term(double s, int q, int k, bool fl
 }
 
 template <int CR, int CC>
-__global__ void __launch_bounds__(256) conjugate_kernel(const ConjugateParams P) {
+__global__ void __launch_bounds__(256) conjugate_kernel(const __grid_constant__ ConjugatePair Q) {
   __shared__ double tile[kWarps][4][72];
+  const ConjugateParams& P = Q.part[blockIdx.z];
   constexpr int BH = 8 * CR, BW = 8 * CC;
   const int lane = threadIdx.x, b = lane >> 3, m = lane & 7;
   const int rows = P.g.rows, columns = P.g.columns, pitch = P.g.pitch;
   const int vbx = blockIdx.x * 4 + b;
-  const int vby = blockIdx.y * kWarps + threadIdx.y;
+  const int vby = blockIdx.y * blockDim.y + threadIdx.y;
   const bool active = vbx * BW < columns && vby * BH < rows;
   const bool in_blocks = active && vby < P.component.block_rows && vbx < P.component.block_columns;
   const int j0 = vbx * BW + m * CC, i0 = vby * BH;
@@ -1397,6 +1374,19 @@ dim3 block_grid(const Geometry& g, const ComponentDevice& c) {
   return dim3((vbc + 3) / 4, (vbr + kWarps - 1) / kWarps, 1);
 }
 
+// The conjugates' CTAs: 8 warps, a block row each, or 2 where those make fewer than 400 CTAs -- a
+// lane's loads are a serial chain, so a small picture's are spread over more SMs (Cb and Cr of
+// 768x512: 48 CTAs of 8 warps, 17.2 us each; in one launch of 2 x 192 CTAs: 13.0 us together).
+dim3 conjugate_grid(const Geometry& g, const ComponentDevice& c, int warps) {
+  const dim3 rows = block_grid(g, c);
+  const int vbr = (g.rows + 8 * c.cell_rows - 1) / (8 * c.cell_rows);
+  return dim3(rows.x, (vbr + warps - 1) / warps, 1);
+}
+int conjugate_warps(const Geometry& g, const ComponentDevice& c) {
+  const dim3 d = block_grid(g, c);
+  return d.x * d.y < 400 ? 2 : kWarps;
+}
+
 template <template <int, int> class Launch, typename... A>
 cudaError_t by_cells(int cr, int cc, A&&... args) {
 #define URB_CELL(R, C) \
@@ -1441,8 +1431,12 @@ struct CanvasLaunch {
 
 template <int CR, int CC>
 struct ConjugateLaunch {
-  static cudaError_t run(const ConjugateParams& p, cudaStream_t s) {
-    conjugate_kernel<CR, CC><<<block_grid(p.g, p.component), dim3(32, kWarps), 0, s>>>(p);
+  static cudaError_t run(const ConjugatePair& q, int count, cudaStream_t s) {
+    const ConjugateParams& p = q.part[0];
+    const int warps = conjugate_warps(p.g, p.component);
+    dim3 grid = conjugate_grid(p.g, p.component, warps);
+    grid.z = count;
+    conjugate_kernel<CR, CC><<<grid, dim3(32, warps), 0, s>>>(q);
     return cudaGetLastError();
   }
 };
@@ -1508,10 +1502,9 @@ int primal_grid_blocks(const Geometry& g, const ComponentDevice& c) {
   const dim3 d = primal_grid(g, c.cell_rows, c.cell_columns);
   return static_cast<int>(d.x * d.y);
 }
-// The conjugate kernel's CTAs (one per block_grid cell: 4 block columns by kWarps block rows),
-// each of which writes one partial sum.
+// The conjugate kernel's CTAs of a component, each of which writes one partial sum.
 int conjugate_grid_blocks(const Geometry& g, const ComponentDevice& c) {
-  const dim3 d = block_grid(g, c);
+  const dim3 d = conjugate_grid(g, c, conjugate_warps(g, c));
   return static_cast<int>(d.x * d.y);
 }
 int start_grid_blocks(const ComponentDevice& c) { return (c.block_rows * c.block_columns * 8 + 255) / 256; }
@@ -1676,8 +1669,10 @@ cudaError_t launch_norms(const NormParams& p, bool tgv, bool coupled, cudaStream
   return tgv ? norms_channels<true>(p, coupled, stream) : norms_channels<false>(p, coupled, stream);
 }
 
-cudaError_t launch_conjugate(const ConjugateParams& p, cudaStream_t stream) {
-  return by_cells<ConjugateLaunch>(p.component.cell_rows, p.component.cell_columns, p, stream);
+cudaError_t launch_conjugate(const ConjugateParams* parts, int count, cudaStream_t stream) {
+  if (count < 1 || count > 2) return cudaErrorInvalidValue;
+  const ConjugatePair pair{{parts[0], parts[count - 1]}};
+  return by_cells<ConjugateLaunch>(parts[0].component.cell_rows, parts[0].component.cell_columns, pair, count, stream);
 }
 
 cudaError_t launch_reductions(const Reductions& r, cudaStream_t stream) {

@@ -335,7 +335,12 @@ cudaError_t launch_gradient(const float* x, float* w1, float* w2, const Geometry
 cudaError_t launch_project(Fields f, const Geometry& g, bool tgv, bool coupled, float radius, float radius0,
                            cudaStream_t stream);
 cudaError_t launch_norms(const NormParams& p, bool tgv, bool coupled, cudaStream_t stream);
-cudaError_t launch_conjugate(const ConjugateParams& p, cudaStream_t stream);
+// G* of 1 or 2 components of the same cells and geometry in one launch; the second's partials follow
+// the first's (parts[0].partials has room for both).
+struct ConjugatePair {
+  ConjugateParams part[2];
+};
+cudaError_t launch_conjugate(const ConjugateParams* parts, int count, cudaStream_t stream);
 cudaError_t launch_residual(const ResidualParams& p, cudaStream_t stream);
 // The dual step as a TMA-fed sweep (sweep.cu): `state` maps the input state's planes (fields x,
 // p1, p2 and for TGV w1, w2, r11, r22, r12, each channel after channel, one allocation), `tilde`
@@ -428,6 +433,8 @@ struct IterationParams {
   ComponentDevice component[kMaxChannels];
   float* next = nullptr;
   int strip_rows = 256;  // rows a CTA sweeps, a multiple of 16 (set by the launcher)
+  float* v = nullptr;    // the walk's, where it keeps its primal step (walk.cuh)
+  double* partials[kMaxChannels] = {};
 };
 
 // Whether the fused sweep takes this canvas: 1 or 3 channels, channel 0 of 1 x 1 cells, the
@@ -439,14 +446,23 @@ bool make_iteration_map(CUtensorMap& map, const float* planes, const Geometry& g
 cudaError_t launch_iteration(const CUtensorMap& state, const CUtensorMap& tilde, const IterationParams& p, bool tgv,
                              bool coupled, int cell_rows, int cell_columns, cudaStream_t stream);
 
-// The same iteration as a walk (walk.cu), which takes what iteration_takes says: the default. Its
+// The same iteration as a walk (walk.cuh), which takes what iteration_takes says: the default. Its
 // map boxes two rows of `count` planes, a state's and behind them those of x~ that its primal step
 // made; `p.next` lies likewise behind p.dual.out.
 // And planes of less than 2^30 samples: offsets within one are 32 bits of bytes.
 inline bool walk_takes(const Geometry& g) { return g.plane < (std::size_t{1} << 30); }
 bool make_walk_map(CUtensorMap& map, const float* planes, const Geometry& g, int count);
+// What a walk keeps for a record: nothing; its primal step's zeta, v and sums of G's terms (each
+// warp's into p.partials, *partials of them a component, at most walk_partials); its dual step's
+// tilde duals.
+enum class WalkKeep { nothing, primal, duals };
+int walk_partials(const Geometry& g);
 cudaError_t launch_walk(const CUtensorMap& map, const IterationParams& p, bool tgv, bool coupled, int cell_rows,
-                        int cell_columns, cudaStream_t stream);
+                        int cell_columns, WalkKeep keep, cudaStream_t stream, int* partials = nullptr);
+cudaError_t launch_walk_primal(const CUtensorMap& map, const IterationParams& p, bool tgv, bool coupled, int cell_rows,
+                               int cell_columns, cudaStream_t stream, int* partials);
+cudaError_t launch_walk_duals(const CUtensorMap& map, const IterationParams& p, bool tgv, bool coupled, int cell_rows,
+                              int cell_columns, cudaStream_t stream);
 
 // Pictures of rounded samples in one sweep per iteration (iteration.cu): the dual step and the
 // next primal step with its sample-by-sample proximal map; maps as make_iteration_map makes them.

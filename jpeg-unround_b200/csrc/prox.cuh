@@ -1,5 +1,6 @@
 // The proximal map of G at one coefficient in binary32 (docs/math.md 4.1, 4.4), shared by the
-// primal-step kernels (kernels.cu) and the fused iteration (iteration.cu).
+// primal-step kernels (kernels.cu), the walk (walk.cuh) and the fused iteration (iteration.cu); and
+// G at a coefficient.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -42,6 +43,30 @@ __device__ __forceinline__ float prox_at(float e, int q, int k, bool flat, const
   const float below = fminf(own_low, z + h);
   const float inside = z < own_low ? below : z;
   return clamp_to(z > own_high ? above : inside, low, high);
+}
+
+// G's terms at a coefficient in binary64 (cpp/src/model.cpp:384-392): m/2 (c - centre)^2, and
+// the cost of lying beyond the file's own interval.
+__device__ __forceinline__ double value_term(double zeta, int q, int k, bool flat, const Constants64& K) {
+  const double level = static_cast<double>(q);
+  const double step = K.step[k];
+  const double shift = k == 0 ? 1024.0 : 0.0;
+  double centre;
+  if (K.mmse && k != 0) {
+    const double size = (fabs(level) - K.shrink[k]) * step;
+    centre = q == 0 ? 0.0 : (q < 0 ? -size : size);
+  } else {
+    centre = level * step + shift;
+  }
+  const double m = flat ? K.flat_weight[k] : K.weight[k];
+  const double away = zeta - centre;
+  double term = 0.5 * m * (away * away);
+  if (K.costed) {
+    const double own_low = (level - 0.5) * step + shift;
+    const double own_high = (level + 0.5) * step + shift;
+    term = term + K.cost[k] * fmax(fmax(zeta - own_high, own_low - zeta), 0.0);
+  }
+  return term;
 }
 
 }  // namespace urb

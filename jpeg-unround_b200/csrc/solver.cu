@@ -20,7 +20,7 @@ std::string describe(cudaError_t error) {
   return std::string(cudaGetErrorName(error)) + ": " + cudaGetErrorString(error);
 }
 
-// How the iterations that keep nothing run: by default as one launch each, the walk of walk.cu
+// How the iterations that keep nothing run: by default as one launch each, the walk of walk.cuh
 // (the dual step and the next primal step, one pass over HBM); with UNROUND_B200_KERNELS=split
 // as the dual sweep and the primal kernels apart, with =fused as the sweep of iteration.cu.
 enum class Kernels { split, fused, walk };
@@ -89,8 +89,18 @@ struct Solver::Impl {
   // x~_{n+1}); `xt` is the current one, xts[xt_id]. The fused sweep's maps, of 9-row boxes.
   float* xts[2] = {nullptr, nullptr};
   int xt_id = 0;
+  // A record on the stream: where its sums lie (first and second reductions), and its marks.
+  struct RecordSums {
+    std::uint64_t iteration = 0;
+    int first = -1, second = -1, most = -1;
+    std::vector<int> data, dual, partial, residual;
+  };
+  RecordSums made;
+  HostBuffer sums;
+  cudaEvent_t loop_begun = nullptr, record_begun = nullptr, record_done = nullptr;
+  const float* record_xt = nullptr;  // x~ of the last dual step: the tilde point's, for its record
   bool fusable = false;
-  bool walks = false;  // fusable, by the walk of walk.cu
+  bool walks = false;  // fusable, by the walk of walk.cuh
   int cell_rows = 1, cell_columns = 1;
   CUtensorMap iteration_state_maps[2];
   CUtensorMap iteration_tilde_maps[2];
@@ -123,6 +133,10 @@ struct Solver::Impl {
 
   ~Impl() {
     if (group_exec != nullptr) cudaGraphExecDestroy(group_exec);
+    cudaStreamSynchronize(stream);  // no copy into `sums` is on its way
+    for (cudaEvent_t e : {loop_begun, record_begun, record_done}) {
+      if (e != nullptr) cudaEventDestroy(e);
+    }
     for (void* p : owned) cudaFreeAsync(p, stream);
     cudaStreamSynchronize(stream);
   }
@@ -148,7 +162,7 @@ struct Solver::Impl {
 
   // A state's fields in one allocation, each field's channels one after another, in the order
   // x, p1, p2, w1, w2, r11, r22, r12: the planes of the sweep's TMA box (sweep.cu).
-  // With `tilde`, x~'s planes lie behind them (the walk's box, walk.cu).
+  // With `tilde`, x~'s planes lie behind them (the walk's box, walk.cuh).
   Fields fields(bool with_tgv, float** tilde = nullptr) {
     const std::size_t n = g.plane * g.channels;
     const int count = with_tgv ? 8 : 3;
@@ -297,7 +311,8 @@ struct Solver::Impl {
     for (const ComponentDevice& d : components) {
       most = std::max<std::size_t>(most, conjugate_grid_blocks(g, d));
       most = std::max<std::size_t>(most, start_grid_blocks(d));
-      const int count = std::max({primal_grid_blocks(g, d), primal_tma_grid_blocks(g, d), start_grid_blocks(d)});
+      const int count = std::max({primal_grid_blocks(g, d), primal_tma_grid_blocks(g, d), start_grid_blocks(d),
+                                  walk_partials(g)});
       value_counts.push_back(count);
       value_written.push_back(0);
     }
@@ -478,6 +493,7 @@ struct Solver::Impl {
       }
     };
     copy(xt, s.x);
+    record_xt = xt;
     copy(tilde.p1, s.p1);
     copy(tilde.p2, s.p2);
     if (tgv) {
@@ -588,6 +604,7 @@ struct Solver::Impl {
   void dual(bool keep) {
     plain_dual = plain_dual || !keep;
     const DualParams dp = dual_params();
+    record_xt = xt;
     if (error == cudaSuccess) {
       error = swept ? launch_dual_tma(state_maps[current], tilde_maps[xt_id], dp, tgv, plan.coupled, keep, stream)
                     : launch_dual(dp, tgv, plan.coupled, keep, stream);
@@ -635,8 +652,9 @@ struct Solver::Impl {
     return error == cudaSuccess;
   }
 
-  void fused() {
-    plain_fused = true;
+  void fused(WalkKeep keep = WalkKeep::nothing) {
+    plain_fused = plain_fused || keep == WalkKeep::nothing;
+    record_xt = xt;
     if (samples != nullptr && samples_layout == 2) {
       SamplesStep q;
       q.levels = s_levels;
@@ -676,10 +694,15 @@ struct Solver::Impl {
     ip.dual = dual_params();
     for (std::size_t c = 0; c < components.size(); ++c) ip.component[c] = components[c];
     ip.next = xts[1 - xt_id];
+    ip.v = v;
+    for (std::size_t c = 0; c < components.size(); ++c) ip.partials[c] = value_slot(c);
     if (error == cudaSuccess) {
-      error = walks ? launch_walk(iteration_state_maps[current], ip, tgv, plan.coupled, cell_rows, cell_columns, stream)
+      int partials = 0;
+      error = walks ? launch_walk(iteration_state_maps[current], ip, tgv, plan.coupled, cell_rows, cell_columns, keep,
+                                  stream, &partials)
                     : launch_iteration(iteration_state_maps[current], iteration_tilde_maps[xt_id], ip, tgv,
                                        plan.coupled, cell_rows, cell_columns, stream);
+      if (keep == WalkKeep::primal) value_written.assign(components.size(), partials);
     }
     current = 1 - current;
     xt_id = 1 - xt_id;
@@ -701,8 +724,10 @@ struct Solver::Impl {
     }
     return conjugate_grid_blocks(g, components[c]);
   }
-  int conjugate_into(std::size_t c, const float* q1, const float* q2, double scale, const double* most_at,
-                     double* out) {
+  // With `pair`, those of channel c + 1 too (of the same cells; q1 and q2 of it `step` floats on),
+  // behind c's: the count of each is returned.
+  int conjugate_into(std::size_t c, const float* q1, const float* q2, double scale, const double* most_at, double* out,
+                     bool pair = false, std::size_t step = 0) {
     if (samples != nullptr) {
       SamplesConjugateParams sp;
       sp.g = g;
@@ -720,20 +745,32 @@ struct Solver::Impl {
       if (error == cudaSuccess) error = launch_samples_conjugate(sp, stream);
       return conjugate_count(c);
     }
-    ConjugateParams cp;
-    cp.g = g;
-    cp.component = components[c];
-    cp.q1 = q1;
-    cp.q2 = q2;
-    cp.scale = scale;
-    cp.most_at = most_at;
-    cp.alpha1 = plan.alpha1;
-    cp.gamma = plan.channel_weights[c];
-    cp.radius = plan.free_radius;
-    cp.free = frame.components[c].free ? 1 : 0;
-    cp.partials = out;
-    if (error == cudaSuccess) error = launch_conjugate(cp, stream);
+    ConjugateParams parts[2];
+    for (std::size_t k = 0; k < (pair ? 2u : 1u); ++k) {
+      ConjugateParams& cp = parts[k];
+      cp.g = g;
+      cp.component = components[c + k];
+      cp.q1 = q1 + k * step;
+      cp.q2 = q2 + k * step;
+      cp.scale = scale;
+      cp.most_at = most_at;
+      cp.alpha1 = plan.alpha1;
+      cp.gamma = plan.channel_weights[c + k];
+      cp.radius = plan.free_radius;
+      cp.free = frame.components[c + k].free ? 1 : 0;
+      cp.partials = out;
+    }
+    if (error == cudaSuccess) error = launch_conjugate(parts, pair ? 2 : 1, stream);
     return conjugate_count(c);
+  }
+
+  // Whether channels c and c + 1 go in one launch of the conjugates.
+  bool conjugate_pair(std::size_t c) const {
+    return samples == nullptr && c + 1 < components.size() &&
+           components[c].cell_rows == components[c + 1].cell_rows &&
+           components[c].cell_columns == components[c + 1].cell_columns &&
+           components[c].block_rows == components[c + 1].block_rows &&
+           components[c].block_columns == components[c + 1].block_columns;
   }
 
   // The channels of the data term: the components, or the samples' channels.
@@ -750,7 +787,7 @@ struct Solver::Impl {
     f.data = data_value();
     NormParams np;
     np.g = g;
-    np.xt = xt;
+    np.xt = record_xt;
     np.tilde = tilde;
     np.div2 = div2;
     for (int c = 0; c < g.channels; ++c) np.weight[c] = plan.channel_weights[c];
@@ -805,14 +842,19 @@ struct Solver::Impl {
   // with no host round trip among them: the norms, then every sum reduced on the device (the
   // norms, the largest |div_2 r~|, the data term of each component), the conjugates at the theta
   // those give (read on the device), their sums, and one copy of the sums to the host.
-  Record record(std::uint64_t iteration) {
-    Record r;
-    r.iteration = iteration;
-    r.scaling = kNaN;
-    r.partial_gap = kNaN;
+  // Its sums come into pinned memory: enqueue_record() puts it on the stream, collect_record() waits
+  // for it, so that the iterations after it can follow on the stream meanwhile.
+  void enqueue_record(std::uint64_t iteration) {
+    if (record_begun == nullptr) {
+      if (error == cudaSuccess) error = cudaEventCreate(&record_begun);
+      if (error == cudaSuccess) error = cudaEventCreate(&record_done);
+    }
+    if (error == cudaSuccess) error = cudaEventRecord(record_begun, stream);
+    made = RecordSums{};
+    made.iteration = iteration;
     NormParams np;
     np.g = g;
-    np.xt = xt;
+    np.xt = record_xt;
     np.tilde = tilde;
     np.div2 = div2;
     for (int c = 0; c < g.channels; ++c) np.weight[c] = plan.channel_weights[c];
@@ -821,15 +863,14 @@ struct Solver::Impl {
     const int count = norms_grid_blocks(g);
     Reductions first;
     first.out = record_sums;
-    const int at_first = first.add(partials, count);
-    const int at_second = tgv ? first.add(partials + count, count) : -1;
-    const int at_most = tgv ? first.add(partials + 2 * count, count, true) : -1;
-    std::vector<int> at_data;
+    made.first = first.add(partials, count);
+    made.second = tgv ? first.add(partials + count, count) : -1;
+    made.most = tgv ? first.add(partials + 2 * count, count, true) : -1;
     if (samples != nullptr) {
-      at_data.push_back(first.add(value_partials, static_cast<int>(samples_written)));
+      made.data.push_back(first.add(value_partials, static_cast<int>(samples_written)));
     } else {
       for (std::size_t c = 0; c < components.size(); ++c) {
-        at_data.push_back(first.add(value_slot(c), static_cast<int>(value_written[c])));
+        made.data.push_back(first.add(value_slot(c), static_cast<int>(value_written[c])));
       }
     }
     if (error == cudaSuccess) error = launch_reductions(first, stream);
@@ -837,19 +878,19 @@ struct Solver::Impl {
     Reductions second;
     second.out = record_sums + kMaxReductions;
     double* region = record_partials;
-    std::vector<int> at_dual, at_partial, at_residual;
-    const double* most_at = tgv ? record_sums + at_most : nullptr;
+    const double* most_at = tgv ? record_sums + made.most : nullptr;
     for (std::size_t c = 0; c < data_channels(); ++c) {
       const float* q1 = tgv ? div2 + 2 * c * g.plane : tilde.p1 + c * g.plane;
       const float* q2 = tgv ? div2 + (2 * c + 1) * g.plane : tilde.p2 + c * g.plane;
-      const int n = conjugate_into(c, q1, q2, 1.0, most_at, region);
-      at_dual.push_back(second.add(region, n));
-      region += n;
+      const bool pair = conjugate_pair(c);
+      const int n = conjugate_into(c, q1, q2, 1.0, most_at, region, pair, (tgv ? 2 : 1) * g.plane);
+      for (int k = 0; k < (pair ? 2 : 1); ++k, region += n) made.dual.push_back(second.add(region, n));
+      if (pair) ++c;
     }
     if (tgv && plan.partial_radius) {
       for (std::size_t c = 0; c < data_channels(); ++c) {
         const int n = conjugate_into(c, tilde.p1 + c * g.plane, tilde.p2 + c * g.plane, 1.0, nullptr, region);
-        at_partial.push_back(second.add(region, n));
+        made.partial.push_back(second.add(region, n));
         region += n;
         ResidualParams rp;
         rp.g = g;
@@ -860,34 +901,47 @@ struct Solver::Impl {
         rp.partials = region;
         if (error == cudaSuccess) error = launch_residual(rp, stream);
         const int residuals = residual_grid_blocks(g);
-        at_residual.push_back(second.add(region, residuals));
+        made.residual.push_back(second.add(region, residuals));
         region += residuals;
       }
     }
     if (error == cudaSuccess) error = launch_reductions(second, stream);
-    double sums[2 * kMaxReductions] = {};
+    sums.resize(2 * kMaxReductions);
     if (error == cudaSuccess) {
-      error = cudaMemcpyAsync(sums, record_sums, sizeof(sums), cudaMemcpyDeviceToHost, stream);
+      error = cudaMemcpyAsync(sums.data(), record_sums, 2 * kMaxReductions * sizeof(double), cudaMemcpyDeviceToHost,
+                              stream);
     }
-    if (error == cudaSuccess) error = cudaStreamSynchronize(stream);
+    if (error == cudaSuccess) error = cudaEventRecord(record_done, stream);
+  }
+
+  Record collect_record() {
+    Record r;
+    r.iteration = made.iteration;
+    r.scaling = kNaN;
+    r.partial_gap = kNaN;
+    if (error == cudaSuccess) error = cudaEventSynchronize(record_done);
+    float milliseconds = 0.0f;  // from the loop's start to the record's
+    if (error == cudaSuccess) error = cudaEventElapsedTime(&milliseconds, loop_begun, record_begun);
     if (error != cudaSuccess) return r;
-    const double* second_sums = sums + kMaxReductions;
+    r.seconds = 1e-3 * static_cast<double>(milliseconds);
+    const double* first_sums = sums.data();
+    const double* second_sums = first_sums + kMaxReductions;
     double data = 0.0;
-    for (int k : at_data) data += sums[k];
+    for (int k : made.data) data += first_sums[k];
     double conjugates = 0.0;
-    for (int k : at_dual) conjugates += second_sums[k];
+    for (int k : made.dual) conjugates += second_sums[k];
     r.dual = -conjugates;
     if (!tgv) {
-      r.primal = plan.alpha * sums[at_first] + data;
+      r.primal = plan.alpha * first_sums[made.first] + data;
       return r;
     }
-    r.primal = (plan.alpha1 * sums[at_first] + plan.alpha0 * sums[at_second]) + data;
-    r.scaling = -negative_theta(sums[at_most], plan.alpha1);
+    r.primal = (plan.alpha1 * first_sums[made.first] + plan.alpha0 * first_sums[made.second]) + data;
+    r.scaling = -negative_theta(first_sums[made.most], plan.alpha1);
     if (plan.partial_radius) {
       double partial = 0.0, residual = 0.0;
-      for (std::size_t c = 0; c < at_partial.size(); ++c) {
-        partial += second_sums[at_partial[c]];
-        residual += plan.channel_weights[c] * second_sums[at_residual[c]];
+      for (std::size_t c = 0; c < made.partial.size(); ++c) {
+        partial += second_sums[made.partial[c]];
+        residual += plan.channel_weights[c] * second_sums[made.residual[c]];
       }
       r.partial_gap = r.primal + partial + *plan.partial_radius * residual;
     }
@@ -1066,17 +1120,15 @@ bool Solver::run(std::uint64_t first, const Observer& observer, Outcome& out, Fa
   const double samples = static_cast<double>(m.g.channels) * m.g.rows * m.g.columns;
   const std::uint64_t most = plan->iterations;
   const std::uint64_t every = plan->record_every;
-  using Clock = std::chrono::steady_clock;
-  const auto began = Clock::now();
-  double recording = 0.0;
   std::int32_t stop = 0;
-  auto take = [&](std::uint64_t iteration) -> bool {
-    const auto at = Clock::now();
-    if (m.error == cudaSuccess) m.error = cudaStreamSynchronize(m.stream);
-    Record r = m.record(iteration);
-    const auto done = Clock::now();
-    recording += std::chrono::duration<double>(done - at).count();
-    r.seconds = std::chrono::duration<double>(at - began).count();
+  if (m.loop_begun == nullptr && m.error == cudaSuccess) m.error = cudaEventCreate(&m.loop_begun);
+  if (m.error == cudaSuccess) m.error = cudaEventRecord(m.loop_begun, m.stream);
+  // The record put on the stream last, once it is there: whether the solve stops at it.
+  bool pending = false;
+  auto settle = [&]() -> bool {
+    if (!pending) return false;
+    pending = false;
+    const Record r = m.collect_record();
     if (m.error != cudaSuccess) return true;
     const double gap = r.primal - r.dual;
     bool met = false;
@@ -1108,6 +1160,14 @@ bool Solver::run(std::uint64_t first, const Observer& observer, Outcome& out, Fa
     return false;
   };
   auto recorded = [&](std::uint64_t n) { return (every > 0 && n % every == 0) || n == most; };
+  // With the walk, the iterations after a record that keep nothing follow it on the stream before it
+  // is looked at: they leave alone what the result is made from (zeta and v of the last kept primal
+  // step). Everything else settles it at once.
+  auto take = [&](std::uint64_t iteration) -> bool {
+    m.enqueue_record(iteration);
+    pending = true;
+    return m.walks && !observer && !recorded(iteration + 1) ? false : settle();
+  };
   auto none_recorded = [&](std::uint64_t from, std::uint64_t to) {
     for (std::uint64_t n = from; n <= to; ++n) {
       if (recorded(n)) return false;
@@ -1120,17 +1180,25 @@ bool Solver::run(std::uint64_t first, const Observer& observer, Outcome& out, Fa
   if (!stopped && first < most) m.primal(recorded(first + 1));
   while (!stopped && iteration < most && m.error == cudaSuccess) {
     const std::uint64_t next = iteration + 1;
+    if (pending && (recorded(next) || recorded(next + 1)) && settle()) {
+      stopped = true;
+      iteration = m.made.iteration;
+      break;
+    }
     // D_next, P_{next+1}, ..., D_{next+G-1}, P_{next+G} (G = kGraphIterations) as one graph when
     // none of them keeps anything.
     if (next + kGraphIterations - 1 < most && none_recorded(next, next + kGraphIterations) && m.group()) {
       iteration = next + kGraphIterations - 1;
       continue;
     }
-    // One sweep for D_next and P_{next+1} when neither keeps anything: no record after the
-    // dual step, none of the next iterate, and a next iteration to make.
-    if (m.fusable && next < most && !recorded(next) && !recorded(next + 1)) {
-      m.fused();
+    // One launch for D_next and P_{next+1} when there is a next iteration to make and neither keeps
+    // anything (no record after the dual step, none of the next iterate), or by the walk when one
+    // of them does.
+    if (m.fusable && next < most && !(recorded(next) && recorded(next + 1)) &&
+        (m.walks || (!recorded(next) && !recorded(next + 1)))) {
+      m.fused(recorded(next) ? WalkKeep::duals : recorded(next + 1) ? WalkKeep::primal : WalkKeep::nothing);
       iteration = next;
+      if (recorded(iteration)) stopped = take(iteration);
       continue;
     }
     if (m.error != cudaSuccess) break;
@@ -1139,7 +1207,10 @@ bool Solver::run(std::uint64_t first, const Observer& observer, Outcome& out, Fa
     if (recorded(iteration)) stopped = take(iteration);
     if (!stopped && iteration < most) m.primal(recorded(iteration + 1));
   }
-  (void)recording;
+  if (settle()) {
+    stopped = true;
+    iteration = m.made.iteration;
+  }
   if (!m.check(failure, "the iterations")) return false;
   out.iterations = iteration;
   out.stop = stopped ? stop : 2;

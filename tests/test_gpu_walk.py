@@ -1,6 +1,7 @@
-"""The walk (walk.cu: an iteration that keeps nothing as one launch) against the dual sweep and the
-primal kernels apart (UNROUND_B200_KERNELS=split): the same operations on the same operands, so
-the canvases, coefficients and records are equal bit for bit. Sizes at the edges of its strips (32
+"""The walk (walk.cuh: an iteration as one launch, keeping nothing or one of its steps' values)
+against the dual sweep and the primal kernels apart (UNROUND_B200_KERNELS=split): the same
+operations on the same operands, so the canvases and coefficients are equal bit for bit; the
+records' sums are of the same terms in another order (binary64: within 1e-12). Sizes at the edges of its strips (32
 columns, 64 with one channel), chunks (8 rows), bands (8 or 16) and of one and several strips of
 rows; every cell layout it takes and one it leaves to the others; radii whose projections go by
 its packed square root and quotient, and by the library's (far from 1)."""
@@ -81,11 +82,43 @@ def test_flat_fields(method):
 
 
 def _compare(image, options, iterations=60):
-    # 24 iterations between records: eager ones, graphs of eight, and the kept ones between.
-    options = [*options, "--iterations", str(iterations), "--tolerance", "0", "--record-every", "25"]
+    # 24 iterations between records: eager ones, graphs of eight, and the kept ones between; or none
+    # between, one and a few, where a record's two launches meet the next one's.
+    for every, count in ((25, iterations), (1, 4), (2, 7), (3, 11)):
+        _compare_every(image, [*options, "--iterations", str(count), "--tolerance", "0", "--record-every", str(every)])
+
+
+def _compare_every(image, options):
     walk, split = _solve(image, options, False), _solve(image, options, True)
     np.testing.assert_array_equal(walk.canvas, split.canvas)
     for a, b in zip(walk.coefficients, split.coefficients):
         np.testing.assert_array_equal(a, b)
-    for name in ("iterations", "primal", "dual", "scaling"):
-        np.testing.assert_array_equal(getattr(walk.result.history, name), getattr(split.result.history, name))
+    a, b = walk.result.history, split.result.history
+    np.testing.assert_array_equal(a.iterations, b.iterations)
+    np.testing.assert_array_equal(a.scaling, b.scaling)
+    scale = np.abs(b.primal).max() + np.abs(b.dual).max()
+    for name in ("primal", "dual", "partial_gap"):
+        np.testing.assert_allclose(getattr(a, name), getattr(b, name), rtol=1e-12, atol=1e-12 * scale)
+
+
+def test_partial_gap():
+    from unround import synthetic
+
+    image = synthetic.colour(61, 77, quality=75, seed=8, noise=3).image
+    _compare(image, ["--method", "tgv", "--partial-radius", "3"])
+
+
+@pytest.mark.parametrize("every", ["1", "2", "7", "10"])
+@pytest.mark.parametrize("method,tolerance", [("tv", "0.02"), ("tgv", "0.2"), ("tgv", "1e9")])
+def test_a_stop(method, tolerance, every):
+    # The iterations that follow a record on the stream before it is looked at leave the result alone.
+    from unround import synthetic
+
+    image = synthetic.colour(96, 80, quality=75, seed=4, noise=2).image
+    options = ["--method", method, "--tolerance", tolerance, "--iterations", "400", "--record-every", every]
+    walk, split = _solve(image, options, False), _solve(image, options, True)
+    assert walk.result.iterations == split.result.iterations < 400
+    assert walk.result.stop == split.result.stop
+    assert len(walk.result.history.iterations) == len(split.result.history.iterations)
+    np.testing.assert_array_equal(walk.canvas, split.canvas)
+    assert (np.diff(walk.result.history.seconds) >= 0).all()
