@@ -1376,7 +1376,7 @@ dim3 block_grid(const Geometry& g, const ComponentDevice& c) {
 
 // The conjugates' CTAs: 8 warps, a block row each, or 2 where those make fewer than 400 CTAs -- a
 // lane's loads are a serial chain, so a small picture's are spread over more SMs (Cb and Cr of
-// 768x512: 48 CTAs of 8 warps, 17.2 us each; in one launch of 2 x 192 CTAs: 13.0 us together).
+// 768x512: 48 CTAs of 8 warps, 17.2 us each; in one launch of 2 x 192 CTAs: 18.3 us together).
 dim3 conjugate_grid(const Geometry& g, const ComponentDevice& c, int warps) {
   const dim3 rows = block_grid(g, c);
   const int vbr = (g.rows + 8 * c.cell_rows - 1) / (8 * c.cell_rows);

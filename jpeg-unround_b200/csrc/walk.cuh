@@ -33,11 +33,13 @@
 // shared memory; they issue at 1.7 an SM and cycle, held by the latency of dependent operations and
 // by instruction fetch, so that code size counts (the edges' tests are folded into addresses, and
 // what is rarely run is not inlined: 4032x3024 TV 331 -> 261 us). Its rows are there when a chunk
-// begins: of 56 looks at the ring, 55 need no wait. Measured, an iteration as graphs of eight,
-// before (two or three launches) and after: TV grey 160x120 12.6 -> 5.0 us, 512^2 13.3 -> 6.2;
-// TGV grey 512^2 18.4 -> 8.6, 1024^2 25.8 -> 17.5, 4096^2 258 -> 211; TGV 4:2:0 768x512 36.7 ->
-// 19.9, 1919x1083 115 -> 97, 4032x3024 563 -> 536; TV 4:2:0 1919x1083 63.2 -> 46.4, 2048^2 101 (two
-// CTAs an SM, a barrier for each tile) -> 86.
+// begins: of 56 looks at the ring, 55 need no wait. A launch's CTAs start on the places that the one
+// before leaves (programmatic dependent launch) and wait for its end with their barriers and
+// factors ready: 1-5 us of an iteration (160x120 5.2 -> 4.4, 2048^2 of three channels 174 -> 168).
+// Measured, an iteration as graphs of eight, before (two or three launches) and after: TV grey
+// 160x120 12.6 -> 4.4 us, 512^2 13.3 -> 5.4; TGV grey 512^2 18.4 -> 8.5, 2048^2 74 -> 66; TGV 4:2:0
+// 768x512 36.7 -> 19.2, 2048^2 200 -> 168; TV 4:2:0 1919x1083 63.2 -> 44.8, 2048^2 101 (two CTAs an
+// SM, a barrier for each tile) -> 85.
 #pragma once
 
 #include <algorithm>
@@ -721,6 +723,9 @@ struct Walk {
         }
       }
     };
+    // Nothing of the state is read or written before the launch before this one is done: every other
+    // warp waits for rows that are copied from here on.
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     issue_to(kSlots);
     if (!left_column(bars, failed, 0, lane)) return false;
     for (int k = 0; k < chunks; ++k) {
@@ -778,6 +783,9 @@ __global__ void __launch_bounds__(walk_threads<C>(), walk_ctas<TGV, C>())
   __shared__ WalkFactors factors[C];
   __shared__ int failed;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  // The next iteration's CTAs may take the places that this one's leave; they wait for its end
+  // (copy_warp) with what does not depend on it done.
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 #pragma unroll
   for (int c = 0; c < C; ++c) {
     const ProxFactors* all = Q.component[c].factors;
@@ -875,8 +883,17 @@ cudaError_t launch_one(const CUtensorMap& map, const IterationParams& p, cudaStr
   q.strip_rows = walk_rows(p.dual.g, ctas, W::WIDTH, 8 * CR);
   const dim3 grid((p.dual.g.columns + W::WIDTH - 1) / W::WIDTH, (p.dual.g.rows + q.strip_rows - 1) / q.strip_rows);
   if (partials != nullptr) *partials = static_cast<int>(grid.x * grid.y) * (C == 1 ? 2 : 1);
-  kernel<<<grid, walk_threads<C>(), bytes, s>>>(map, q);
-  return cudaGetLastError();
+  cudaLaunchConfig_t config = {};
+  config.gridDim = grid;
+  config.blockDim = dim3(walk_threads<C>());
+  config.dynamicSmemBytes = bytes;
+  config.stream = s;
+  cudaLaunchAttribute early;
+  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  early.val.programmaticStreamSerializationAllowed = 1;
+  config.attrs = &early;
+  config.numAttrs = 1;
+  return cudaLaunchKernelEx(&config, kernel, map, q);
 }
 
 template <bool TGV, bool COUPLED, int KEEP>
