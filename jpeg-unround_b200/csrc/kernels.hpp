@@ -464,6 +464,27 @@ cudaError_t launch_walk_primal(const CUtensorMap& map, const IterationParams& p,
 cudaError_t launch_walk_duals(const CUtensorMap& map, const IterationParams& p, bool tgv, bool coupled, int cell_rows,
                               int cell_columns, cudaStream_t stream);
 
+// The unrolled solve's iteration (walk_unrolled.cu): the dual step D_k from s_{k-1} and x~_k and the
+// primal step P_{k+1}, of every picture at once, each with its own parameters. The planes of a
+// state, and of x~ behind them, are `images` pictures of rows x columns (whole 8 x 8 blocks),
+// packed; the map boxes 72 columns x 2 rows of one picture of the 9 planes (make_fields_map).
+struct UnrolledWalk {
+  IterationParams step;  // dual.g (a picture's rows, columns, pitch = columns), out, rho, rest; next
+  int images = 0;
+  const float* lower = nullptr;   // [image][block][64], the DC interval centred on its middle
+  const float* upper = nullptr;
+  const float* centre = nullptr;
+  const float* middle = nullptr;  // [image][block]
+  const float* weight = nullptr;  // [image][64]
+  const float* flat_weight = nullptr;
+  const std::uint8_t* flat = nullptr;  // [image][block]
+  const float* alpha0 = nullptr;       // [image]
+  const float* alpha1 = nullptr;
+  const float* tau = nullptr;
+  const float* sigma = nullptr;
+};
+cudaError_t launch_walk_unrolled(const CUtensorMap& map, const UnrolledWalk& p, cudaStream_t stream);
+
 // Pictures of rounded samples in one sweep per iteration (iteration.cu): the dual step and the
 // next primal step with its sample-by-sample proximal map; maps as make_iteration_map makes them.
 struct SamplesIterationParams {

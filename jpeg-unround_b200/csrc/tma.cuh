@@ -55,6 +55,16 @@ __device__ __forceinline__ void load_box(float* to, const CUtensorMap* map, std:
       : "memory");
 }
 
+// A box of one picture (`z`) of the planes of a 4D map (make_fields_map), every field.
+__device__ __forceinline__ void load_fields(float* to, const CUtensorMap* map, std::uint64_t* bar, int x, int y,
+                                            int z) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, "
+      "%5}], [%6];" ::"r"(smem_address(to)),
+      "l"(map), "r"(x), "r"(y), "r"(z), "r"(0), "r"(smem_address(bar))
+      : "memory");
+}
+
 // A contiguous bulk copy of `bytes` (a multiple of 16; both addresses 16-byte aligned) from
 // global into shared memory, completing on `bar`.
 __device__ __forceinline__ void load_bulk(void* to, const void* from, unsigned bytes, std::uint64_t* bar) {

@@ -12,8 +12,8 @@
 // a, b) with t = tau m_k (m_k the data term's weight of frequency k, of a flat block where the
 // block is flat) and e the DCT of the block less the middle of its DC interval.
 //
-// P_k is a block kernel (a warp per block row, the transforms in registers); D_k a tile kernel
-// fed by a bulk-tensor copy of s_{k-1} and x~_k with halos.
+// P_1 is a block kernel (a warp per block row, the transforms in registers); D_k and P_{k+1} after
+// it one launch, the walk of walk_unrolled.cu.
 //
 // The adjoint runs the iterations backwards: the adjoint of D_k (one tile kernel: the
 // projections' Jacobians, then the transposes of E, grad and div2 over the tile, from shared
@@ -34,6 +34,7 @@
 
 #include "dct.cuh"
 #include "kernels.hpp"
+#include "tma.cuh"
 #include "unround.h"
 #include "unround_b200.h"
 
@@ -74,11 +75,6 @@ struct Problem {
 
 __device__ __forceinline__ std::size_t at(const Problem& q, int z, int i, int j) {
   return (static_cast<std::size_t>(z) * q.rows + i) * q.columns + j;
-}
-
-__device__ __forceinline__ float ball(float square, float radius) {
-  const float norm = sqrtf(square);
-  return norm > radius ? radius / norm : 1.0f;
 }
 
 // Sums of a value over a CTA of 256 threads, added to a binary64 total.
@@ -262,32 +258,6 @@ static_assert(kStateFloats % 32 == 0, "the adjoint's box starts 128-byte aligned
 constexpr std::size_t kAdjointShared =
     static_cast<std::size_t>(kStateFloats + kBarFloats + kTildeFloats + kPointFloats) * sizeof(float);
 
-__device__ __forceinline__ unsigned shared_address(const void* p) {
-  return static_cast<unsigned>(__cvta_generic_to_shared(p));
-}
-
-__device__ __forceinline__ void load_fields(float* to, const CUtensorMap* map, std::uint64_t* bar, int x, int y,
-                                            int z) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, "
-      "%5}], [%6];" ::"r"(shared_address(to)),
-      "l"(map), "r"(x), "r"(y), "r"(z), "r"(0), "r"(shared_address(bar))
-      : "memory");
-}
-
-__device__ __forceinline__ bool wait_phase(std::uint64_t* bar, unsigned parity) {
-  for (long long n = 0; n < (1LL << 22); ++n) {
-    unsigned done;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(done)
-        : "r"(shared_address(bar)), "r"(parity)
-        : "memory");
-    if (done != 0) return true;
-  }
-  return false;
-}
-
 __global__ void __launch_bounds__(256) dual_adjoint_kernel(const __grid_constant__ CUtensorMap state_map,
                                                            const __grid_constant__ CUtensorMap bar_map, Problem q,
                                                            Planes b, float* xt_bar, double* grads) {
@@ -303,18 +273,18 @@ __global__ void __launch_bounds__(256) dual_adjoint_kernel(const __grid_constant
   const float rho = q.rho, rest = 1.0f - q.rho, tau = q.tau[z], sigma = q.sigma[z];
   const float alpha0 = q.alpha0[z], alpha1 = q.alpha1[z];
   if (tid == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(shared_address(&loaded[0])) : "memory");
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(shared_address(&loaded[1])) : "memory");
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_address(&loaded[0])) : "memory");
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_address(&loaded[1])) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
   // Two copies on two barriers: (1) needs only the first, which lands while the second is
   // still on its way.
   if (tid == 0) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(shared_address(&loaded[0])),
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_address(&loaded[0])),
                  "r"(static_cast<unsigned>(kStateFloats * sizeof(float)))
                  : "memory");
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(shared_address(&loaded[1])),
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_address(&loaded[1])),
                  "r"(static_cast<unsigned>(kBarFloats * sizeof(float)))
                  : "memory");
     load_fields(S, &state_map, &loaded[0], j0 - 4, i0 - 2, z);
@@ -325,11 +295,11 @@ __global__ void __launch_bounds__(256) dual_adjoint_kernel(const __grid_constant
   auto give_up = [&]() {
     if (tid == 0) {
       atomicAdd(grads + 3 * q.images + z, static_cast<double>(__int_as_float(0x7fc00000)));
-      wait_phase(&loaded[0], 0);
-      wait_phase(&loaded[1], 0);
+      barrier_wait(&loaded[0], 0);
+      barrier_wait(&loaded[1], 0);
     }
   };
-  const bool ready = wait_phase(&loaded[0], 0);
+  const bool ready = barrier_wait(&loaded[0], 0);
   if (__syncthreads_or(!ready)) {
     give_up();
     return;
@@ -363,7 +333,7 @@ __global__ void __launch_bounds__(256) dual_adjoint_kernel(const __grid_constant
       t_at(0, i, j) = 2.0f * tilde1 - w1;
       t_at(1, i, j) = 2.0f * tilde2 - w2;
     }
-    const bool adjoint_ready = wait_phase(&loaded[1], 0);
+    const bool adjoint_ready = barrier_wait(&loaded[1], 0);
     if (__syncthreads_or(!adjoint_ready)) {
       failed = true;
       return;
@@ -525,106 +495,6 @@ __global__ void __launch_bounds__(256) dual_adjoint_kernel(const __grid_constant
   add_sum(g_sigma, grads + 3 * q.images + z);
 }
 
-// The dual step D_k as tiles of 16 rows x 32 columns: s_{k-1} and x~_k (9 planes) with a halo
-// of a row above and below and 4 columns each side by one 4D bulk-tensor copy, w~ over the tile
-// and the column to its left and the row above it in shared memory, then each pixel's step:
-// x- = 2 x~ - x, w- = 2 w~ - w, the points q and s and their projections, and the relaxation.
-constexpr int kForwardRows = kAdjointRows + 2;  // rows i0 - 1 .. i0 + 16
-constexpr int kForwardFloats = kFields * kForwardRows * kAdjointSpan;
-constexpr int kForwardTildeRows = kAdjointRows + 1, kForwardTildeColumns = 33;
-constexpr int kForwardTildeFloats = 2 * kForwardTildeRows * kAdjointSpan;  // rows of kAdjointSpan, as the box
-constexpr std::size_t kForwardShared = static_cast<std::size_t>(kForwardFloats + kForwardTildeFloats) * sizeof(float);
-
-__global__ void __launch_bounds__(256) dual_tile_kernel(const __grid_constant__ CUtensorMap state_map, Problem q,
-                                                        Planes out) {
-  extern __shared__ __align__(128) float shared[];
-  __shared__ __align__(8) std::uint64_t loaded;
-  float* const S = shared;                    // [field][row][column], row i0 - 1 + r, column j0 - 4 + c
-  float* const T = S + kForwardFloats;        // w~, row i0 - 1 + r, column j0 - 1 + c
-  const int lane = threadIdx.x, warp = threadIdx.y, tid = warp * 32 + lane;
-  const int z = blockIdx.z, i0 = blockIdx.y * kAdjointRows, j0 = blockIdx.x * 32;
-  const int H = q.rows, W = q.columns;
-  const float rho = q.rho, rest = 1.0f - q.rho, tau = q.tau[z], sigma = q.sigma[z];
-  const float alpha0 = q.alpha0[z], alpha1 = q.alpha1[z];
-  if (tid == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(shared_address(&loaded)) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  __syncthreads();
-  if (tid == 0) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(shared_address(&loaded)),
-                 "r"(static_cast<unsigned>(kForwardFloats * sizeof(float)))
-                 : "memory");
-    load_fields(S, &state_map, &loaded, j0 - 4, i0 - 1, z);
-  }
-  const bool ready = wait_phase(&loaded, 0);
-  if (__syncthreads_or(!ready)) {
-    // The load did not land: the tile's x is not a number, and no copy may still be writing
-    // into the CTA's shared memory when it leaves.
-    for (int rr = warp; rr < kAdjointRows; rr += 8) {
-      const int i = i0 + rr, j = j0 + lane;
-      if (i < H && j < W) out.x[at(q, z, i, j)] = __int_as_float(0x7fc00000);
-    }
-    if (tid == 0) wait_phase(&loaded, 0);
-    return;
-  }
-  auto s_at = [&](int f, int i, int j) -> float { return S[(f * kForwardRows + i - i0 + 1) * kAdjointSpan + j - j0 + 4]; };
-  auto t_at = [&](int f, int i, int j) -> float& { return T[(f * kForwardTildeRows + i - i0 + 1) * kAdjointSpan + j - j0 + 1]; };
-  enum { X = 0, P1, P2, W1, W2, R11, R22, R12, XT };
-  // w~ = w + tau (p + div2 r), div2 r by forward differences.
-  for (int n = tid; n < kForwardTildeRows * kAdjointSpan; n += 256) {
-    if (n % kAdjointSpan >= kForwardTildeColumns) continue;
-    const int i = i0 - 1 + n / kAdjointSpan, j = j0 - 1 + n % kAdjointSpan;
-    const float r11 = s_at(R11, i, j), r22 = s_at(R22, i, j), r12 = s_at(R12, i, j);
-    float d1 = j + 1 < W ? s_at(R11, i, j + 1) - r11 : 0.0f;
-    float d2 = j + 1 < W ? s_at(R12, i, j + 1) - r12 : 0.0f;
-    d1 = d1 + (i + 1 < H ? s_at(R12, i + 1, j) - r12 : 0.0f);
-    d2 = d2 + (i + 1 < H ? s_at(R22, i + 1, j) - r22 : 0.0f);
-    t_at(0, i, j) = s_at(W1, i, j) + tau * (s_at(P1, i, j) + d1);
-    t_at(1, i, j) = s_at(W2, i, j) + tau * (s_at(P2, i, j) + d2);
-  }
-  __syncthreads();
-  for (int rr = warp; rr < kAdjointRows; rr += 8) {
-    const int i = i0 + rr, j = j0 + lane;
-    if (i >= H || j >= W) continue;
-    const bool right = j + 1 < W, down = i + 1 < H;
-    const float xt = s_at(XT, i, j), x = s_at(X, i, j);
-    const float bar = 2.0f * xt - x;
-    const float g1 = right ? (2.0f * s_at(XT, i, j + 1) - s_at(X, i, j + 1)) - bar : 0.0f;
-    const float g2 = down ? (2.0f * s_at(XT, i + 1, j) - s_at(X, i + 1, j)) - bar : 0.0f;
-    const float t1 = t_at(0, i, j), t2 = t_at(1, i, j), w1 = s_at(W1, i, j), w2 = s_at(W2, i, j);
-    const float b1 = 2.0f * t1 - w1, b2 = 2.0f * t2 - w2;
-    const float p1 = s_at(P1, i, j), p2 = s_at(P2, i, j);
-    const float q1 = p1 + sigma * (g1 - b1);
-    const float q2 = p2 + sigma * (g2 - b2);
-    float l1 = 0.0f, l2 = 0.0f, u1 = 0.0f, u2 = 0.0f;
-    if (j > 0) {
-      l1 = 2.0f * t_at(0, i, j - 1) - s_at(W1, i, j - 1);
-      l2 = 2.0f * t_at(1, i, j - 1) - s_at(W2, i, j - 1);
-    }
-    if (i > 0) {
-      u1 = 2.0f * t_at(0, i - 1, j) - s_at(W1, i - 1, j);
-      u2 = 2.0f * t_at(1, i - 1, j) - s_at(W2, i - 1, j);
-    }
-    const float own1x = right ? b1 : 0.0f, own2x = right ? b2 : 0.0f;
-    const float own1y = down ? b1 : 0.0f, own2y = down ? b2 : 0.0f;
-    const float e11 = own1x - l1, e22 = own2y - u2, e12 = 0.5f * ((own1y - u1) + (own2x - l2));
-    const float r11 = s_at(R11, i, j), r22 = s_at(R22, i, j), r12 = s_at(R12, i, j);
-    const float s11 = r11 + sigma * e11, s22 = r22 + sigma * e22, s12 = r12 + sigma * e12;
-    const float sp = ball(q1 * q1 + q2 * q2, alpha1);
-    const float sr = ball(s11 * s11 + s22 * s22 + 2.0f * (s12 * s12), alpha0);
-    const std::size_t k = at(q, z, i, j);
-    out.x[k] = rho * xt + rest * x;
-    out.p1[k] = rho * (q1 * sp) + rest * p1;
-    out.p2[k] = rho * (q2 * sp) + rest * p2;
-    out.w1[k] = rho * t1 + rest * w1;
-    out.w2[k] = rho * t2 + rest * w2;
-    out.r11[k] = rho * (s11 * sr) + rest * r11;
-    out.r22[k] = rho * (s22 * sr) + rest * r22;
-    out.r12[k] = rho * (s12 * sr) + rest * r12;
-  }
-}
-
 // The primal step's adjoint, per block: from the adjoint of x~ (`xt_bar`) the adjoint of v.
 // x~ = C^T zeta C + middle and e = C (v - middle) C^T, so zeta^ = C x~^ C^T and v^ = C^T e^ C.
 __global__ void __launch_bounds__(256) primal_adjoint_block(Problem q, Planes s, const float* xt_bar, float* vbar,
@@ -717,14 +587,47 @@ dim3 block_grid(const Problem& q) {
   return dim3((q.columns + 31) / 32, (q.blocks_down + 7) / 8, q.images);
 }
 
-// The tiled dual step's and its adjoint's grid: a CTA a tile of kAdjointRows x 32.
+// The dual step's adjoint's grid: a CTA a tile of kAdjointRows x 32.
 dim3 tile_grid(const Problem& q) {
   return dim3((q.columns + 31) / 32, (q.rows + kAdjointRows - 1) / kAdjointRows, q.images);
 }
 
-// The map of 9 planes (a state and the x~ after it) for the tiled dual step.
+// The map of 9 planes (a state and the x~ after it) for the walk.
 bool make_forward_map(CUtensorMap& map, const float* base, const Problem& q) {
-  return make_fields_map(map, base, q.columns, q.rows, q.images, 9, q.plane, kAdjointSpan, kForwardRows);
+  return make_fields_map(map, base, q.columns, q.rows, q.images, 9, q.plane, sweep_width(1) + 8, 2);
+}
+
+// D_k and P_{k+1}: from the 9 planes of `from` (s_{k-1} and x~_k) to s_k at `to` and x~_{k+1} at `next`.
+cudaError_t walk(const CUtensorMap& from, const Problem& q, float* to, float* next, cudaStream_t stream) {
+  UnrolledWalk w;
+  DualParams& d = w.step.dual;
+  d.g.rows = q.rows;
+  d.g.columns = d.g.pitch = q.columns;
+  d.g.plane = q.plane;
+  d.out = Fields{to,
+                 to + q.plane,
+                 to + 2 * q.plane,
+                 to + 3 * q.plane,
+                 to + 4 * q.plane,
+                 to + 5 * q.plane,
+                 to + 6 * q.plane,
+                 to + 7 * q.plane};
+  d.rho = q.rho;
+  d.rest = 1.0f - q.rho;
+  w.step.next = next;
+  w.images = q.images;
+  w.lower = q.lower;
+  w.upper = q.upper;
+  w.centre = q.centre;
+  w.middle = q.middle;
+  w.weight = q.weight;
+  w.flat_weight = q.flat_weight;
+  w.flat = q.flat;
+  w.alpha0 = q.alpha0;
+  w.alpha1 = q.alpha1;
+  w.tau = q.tau;
+  w.sigma = q.sigma;
+  return launch_walk_unrolled(from, w, stream);
 }
 
 std::string check(const unround_b200_unrolled* u) {
@@ -810,7 +713,7 @@ extern "C" unround_status unround_b200_unrolled_forward(const unround_b200_unrol
   const std::size_t plane = q.plane;
   const std::uint64_t n = problem->iterations, every = problem->checkpoint_every;
   float* const spare[2] = {workspace, workspace + 9 * plane};
-  // The dual steps read the 9 planes of s_{k-1} and x~_k by bulk-tensor copies: a map of each
+  // The walks read the 9 planes of s_{k-1} and x~_k by bulk-tensor copies: a map of each
   // checkpoint and of each spare.
   const std::uint64_t segments = urb::checkpoints_of(*problem);
   std::vector<CUtensorMap> checkpoint_maps(segments);
@@ -824,31 +727,30 @@ extern "C" unround_status unround_b200_unrolled_forward(const unround_b200_unrol
     urb::tell(message, message_size, "the device's bulk-tensor copies could not be set up for the dual steps");
     return UNROUND_ERROR_INTERNAL;
   }
-  const dim3 grid = urb::pixel_grid(q), block(32, 8), tiles = urb::tile_grid(q);
+  const dim3 grid = urb::pixel_grid(q), block(32, 8);
   // s_{k-1} and then x~_k live at `current`: 9 planes.
   float* current = checkpoints;
   const CUtensorMap* current_map = &checkpoint_maps[0];
   urb::start_kernel<<<grid, block, 0, on>>>(q, problem->start, urb::planes_of(current, plane));
-  for (std::uint64_t k = 1; k <= n; ++k) {
-    urb::primal_kernel<<<urb::block_grid(q), block, 0, on>>>(q, urb::planes_of(current, plane),
-                                                              k == n ? output : current + 8 * plane);
-    if (k < n) {
-      float* next;
-      const CUtensorMap* next_map;
-      if (k % every == 0) {
-        next = checkpoints + k / every * 9 * plane;
-        next_map = &checkpoint_maps[k / every];
-      } else {
-        const int c = current == spare[0] ? 1 : 0;
-        next = spare[c];
-        next_map = &spare_maps[c];
-      }
-      urb::dual_tile_kernel<<<tiles, block, urb::kForwardShared, on>>>(*current_map, q, urb::planes_of(next, plane));
-      current = next;
-      current_map = next_map;
+  urb::primal_kernel<<<urb::block_grid(q), block, 0, on>>>(q, urb::planes_of(current, plane),
+                                                            n == 1 ? output : current + 8 * plane);
+  cudaError_t error = cudaSuccess;
+  for (std::uint64_t k = 1; k < n && error == cudaSuccess; ++k) {
+    float* next;
+    const CUtensorMap* next_map;
+    if (k % every == 0) {
+      next = checkpoints + k / every * 9 * plane;
+      next_map = &checkpoint_maps[k / every];
+    } else {
+      const int c = current == spare[0] ? 1 : 0;
+      next = spare[c];
+      next_map = &spare_maps[c];
     }
+    error = urb::walk(*current_map, q, next, k + 1 == n ? output : next + 8 * plane, on);
+    current = next;
+    current_map = next_map;
   }
-  const cudaError_t error = cudaGetLastError();
+  if (error == cudaSuccess) error = cudaGetLastError();
   if (error != cudaSuccess) {
     urb::tell(message, message_size, std::string("the device failed in the unrolled solve: ") + cudaGetErrorString(error));
     return UNROUND_ERROR_INTERNAL;
@@ -884,8 +786,8 @@ extern "C" unround_status unround_b200_unrolled_backward(const unround_b200_unro
   auto storage_of = [&](std::uint64_t seg, std::uint64_t step) -> float* {
     return step == 0 ? const_cast<float*>(checkpoints) + seg * 9 * plane : recomputed + (step - 1) * 9 * plane;
   };
-  // The dual step and its adjoint read the 9 planes of each by bulk-tensor copies (boxes of
-  // different heights).
+  // The walk and the dual step's adjoint read the 9 planes of each by bulk-tensor copies (boxes of
+  // different sizes).
   std::vector<CUtensorMap> checkpoint_maps(segments), recomputed_maps(every > 1 ? every - 1 : 0);
   std::vector<CUtensorMap> checkpoint_forward(segments), recomputed_forward(every > 1 ? every - 1 : 0);
   CUtensorMap bar_maps[2];
@@ -911,27 +813,17 @@ extern "C" unround_status unround_b200_unrolled_backward(const unround_b200_unro
   cudaMemsetAsync(grads, 0, 4 * problem->images * sizeof(double), on);
   // The adjoint of s_N's predecessor starts at zero; that of x~_N is the output's gradient.
   int current = 0;
+  cudaError_t error = cudaSuccess;
   cudaMemsetAsync(adjoint[current], 0, 9 * plane * sizeof(float), on);
   cudaMemcpyAsync(xt_bar, output_grad, plane * sizeof(float), cudaMemcpyDeviceToDevice, on);
   for (std::uint64_t seg = segments; seg-- > 0;) {
     const std::uint64_t k0 = seg * every;                             // the checkpoint s_{k0}
     const std::uint64_t k1 = std::min<std::uint64_t>(k0 + every, n);  // the segment's iterations k0+1 .. k1
-    // Recompute s_{k0+1} .. s_{k1-1} and x~_{k0+2} .. x~_{k1} (x~_{k0+1} is the checkpoint's;
-    // x~_N is not needed: x~_bar starts there).
-    for (std::uint64_t k = k0 + 1; k < k1; ++k) {
+    // Recompute s_{k0+1} .. s_{k1-1} and x~_{k0+2} .. x~_{k1} (x~_{k0+1} is the checkpoint's).
+    for (std::uint64_t k = k0 + 1; k < k1 && error == cudaSuccess; ++k) {
       const std::uint64_t step = k - 1 - k0;  // s_{k-1} is storage_of(seg, step)
-      float* from = storage_of(seg, step);
-      if (step > 0) {
-        urb::primal_kernel<<<urb::block_grid(q), block, 0, on>>>(q, urb::planes_of(from, plane), from + 8 * plane);
-      }
-      const CUtensorMap& from_map = step == 0 ? checkpoint_forward[seg] : recomputed_forward[step - 1];
-      urb::dual_tile_kernel<<<tiles, block, urb::kForwardShared, on>>>(from_map, q,
-                                                                       urb::planes_of(storage_of(seg, step + 1), plane));
-    }
-    if (k1 - k0 > 1 && k1 < n) {
-      // x~_{k1} of the segment's last state, for D_{k1}'s adjoint.
-      float* last = storage_of(seg, k1 - 1 - k0);
-      urb::primal_kernel<<<urb::block_grid(q), block, 0, on>>>(q, urb::planes_of(last, plane), last + 8 * plane);
+      float* const to = storage_of(seg, step + 1);
+      error = urb::walk(step == 0 ? checkpoint_forward[seg] : recomputed_forward[step - 1], q, to, to + 8 * plane, on);
     }
     // Backwards through the segment: at iteration k, D_k (k < N) then P_k.
     for (std::uint64_t k = k1; k > k0; --k) {
@@ -950,7 +842,7 @@ extern "C" unround_status unround_b200_unrolled_backward(const unround_b200_unro
           q, urb::planes_of(storage_of(seg, step), plane), xt_bar, adjoint[current] + 8 * plane, grads);
     }
   }
-  const cudaError_t error = cudaGetLastError();
+  if (error == cudaSuccess) error = cudaGetLastError();
   if (error != cudaSuccess) {
     urb::tell(message, message_size, std::string("the device failed in the adjoint: ") + cudaGetErrorString(error));
     return UNROUND_ERROR_INTERNAL;

@@ -88,13 +88,13 @@ __device__ __forceinline__ Pair pair(float x, float y) {
 }
 __device__ __forceinline__ Pair pair(float x) { return pair(x, x); }
 __device__ __forceinline__ float first(Pair p) {
-  float x, y;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(p));
+  float x;
+  asm("{\n .reg .f32 y;\n mov.b64 {%0, y}, %1;\n}\n" : "=f"(x) : "l"(p));
   return x;
 }
 __device__ __forceinline__ float second(Pair p) {
-  float x, y;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(p));
+  float y;
+  asm("{\n .reg .f32 x;\n mov.b64 {x, %0}, %1;\n}\n" : "=f"(y) : "l"(p));
   return y;
 }
 __device__ __forceinline__ Pair add2(Pair a, Pair b) {
@@ -380,18 +380,33 @@ __device__ __noinline__ void general_row(float (&coef)[8], int4 levels, int m, b
   }
 }
 
-template <bool TGV, int C, bool COUPLED, int CR, int CC, int KEEP>
+template <bool TGV, int C, bool COUPLED, int CR, int CC, int KEEP, bool UNROLLED = false>
 struct Walk {
   using W = WalkLayout<TGV, C, CR>;
   static constexpr int L = W::L, SPAN = W::SPAN, WIDTH = W::WIDTH, XS = WIDTH + 4;
   // One channel's kernels of sweep.cu relax p and r, and take the square of p, with the other
   // product fused.
   static constexpr bool REST_FIRST = C == 1;
-  static constexpr bool SQUARE_2 = TGV && C == 1;
+  static constexpr bool SQUARE_2 = TGV && C == 1 && !UNROLLED;
+  // The unrolled solve's kernels relax w with the first product fused.
+  static constexpr bool REST_FIRST_W = !UNROLLED;
 
   const IterationParams& Q;
   float* const shared;
   const int x0, i0, i1;
+  // Of the unrolled solve: the picture, and its parameters (UnrolledWalk).
+  const int image = 0;
+  const float image_tau = 0.0f, image_sigma = 0.0f, image_alpha1 = 0.0f, image_alpha0 = 0.0f;
+
+  __device__ __forceinline__ float tau(int c) const { return UNROLLED ? image_tau : Q.dual.tau[c]; }
+  __device__ __forceinline__ float sigma(int c) const { return UNROLLED ? image_sigma : Q.dual.sigma[c]; }
+  __device__ __forceinline__ float radius() const { return UNROLLED ? image_alpha1 : Q.dual.radius; }
+  __device__ __forceinline__ float radius0() const { return UNROLLED ? image_alpha0 : Q.dual.radius0; }
+  // Row i of the picture among the rows of a plane; an offset within a plane in bytes.
+  using Offset = std::conditional_t<UNROLLED, std::size_t, unsigned>;
+  __device__ __forceinline__ Offset plane_row(int i) const {
+    return UNROLLED ? static_cast<Offset>(image) * Q.dual.g.rows + i : static_cast<Offset>(i);
+  }
 
   // A plane of a slot: a field's, or x~'s.
   static __device__ __forceinline__ int at(int field, int c) { return (field * C + c) * W::PLANE; }
@@ -414,7 +429,7 @@ struct Walk {
     const int o = kHalo + 32 * part + across, j = x0 + 32 * part + across;
     const bool valid = j < P.g.columns;  // the pair (the columns are even)
     const int next = j + 2 < P.g.columns ? o + 2 : o + 1;
-    const unsigned here = (static_cast<unsigned>(FIRST ? 0 : i) * P.g.pitch + j) * 4u;
+    const Offset here = (plane_row(FIRST ? 0 : i) * P.g.pitch + j) * 4u;
     const Pair rho = pair(P.rho), rest = pair(P.rest), minus_two = pair(-2.0f);
     auto own_at = [&](int offset) -> Pair { return *reinterpret_cast<const Pair*>(own + offset + o); };
     auto right_of = [&](int offset, Pair p) -> Pair { return pair(second(p), own[offset + next]); };
@@ -437,13 +452,13 @@ struct Walk {
       put(P.out.x, c, k.xn[c]);
       old_p1[c] = own_at(at(1, c));
       old_p2[c] = own_at(at(2, c));
-      const Pair sigma = pair(P.sigma[c]);
+      const Pair sigma_c = pair(sigma(c));
       if constexpr (!TGV) {
-        step_p1[c] = fma2(sigma, gx, old_p1[c]);
-        step_p2[c] = fma2(sigma, gy, old_p2[c]);
+        step_p1[c] = fma2(sigma_c, gx, old_p1[c]);
+        step_p2[c] = fma2(sigma_c, gy, old_p2[c]);
       } else {
         // w~ = w + tau (p + div2 r), -w-.
-        const Pair tau = pair(P.tau[c]);
+        const Pair tau_c = pair(tau(c));
         const Pair r11 = own_at(at(5, c)), r22 = own_at(at(6, c)), r12 = own_at(at(7, c));
         k.r11[c] = r11;
         k.r22[c] = r22;
@@ -451,24 +466,24 @@ struct Walk {
         const Pair d1 = add2(sub2(right_of(at(5, c), r11), r11), sub2(down_at(at(7, c)), r12));
         const Pair d2 = add2(sub2(right_of(at(7, c), r12), r12), sub2(down_at(at(6, c)), r22));
         const Pair w1 = own_at(at(3, c)), w2 = own_at(at(4, c));
-        const Pair t1 = fma2(tau, add2(old_p1[c], d1), w1), t2 = fma2(tau, add2(old_p2[c], d2), w2);
-        put(P.out.w1, c, fma2(rest, w1, mul2(rho, t1)));
-        put(P.out.w2, c, fma2(rest, w2, mul2(rho, t2)));
+        const Pair t1 = fma2(tau_c, add2(old_p1[c], d1), w1), t2 = fma2(tau_c, add2(old_p2[c], d2), w2);
+        put(P.out.w1, c, REST_FIRST_W ? fma2(rest, w1, mul2(rho, t1)) : fma2(rho, t1, mul2(rest, w1)));
+        put(P.out.w2, c, REST_FIRST_W ? fma2(rest, w2, mul2(rho, t2)) : fma2(rho, t2, mul2(rest, w2)));
         if constexpr (KEEP == 2) {
           put(P.tilde.w1, c, t1);
           put(P.tilde.w2, c, t2);
         }
         k.nb1[c] = fma2(t1, minus_two, w1);
         k.nb2[c] = fma2(t2, minus_two, w2);
-        step_p1[c] = fma2(sigma, add2(gx, k.nb1[c]), old_p1[c]);
-        step_p2[c] = fma2(sigma, add2(gy, k.nb2[c]), old_p2[c]);
+        step_p1[c] = fma2(sigma_c, add2(gx, k.nb1[c]), old_p1[c]);
+        step_p2[c] = fma2(sigma_c, add2(gy, k.nb2[c]), old_p2[c]);
       }
       if constexpr (COUPLED) {
         const Pair square = fma2(step_p1[c], step_p1[c], mul2(step_p2[c], step_p2[c]));
         square_p = c == 0 ? square : add2(square_p, square);
       }
     }
-    const Ball unit(P.radius);
+    const Ball unit(radius());
     Pair scale = 0;
     if constexpr (COUPLED) scale = ball2(square_p, unit);
 #pragma unroll
@@ -508,7 +523,7 @@ struct Walk {
     const bool has_down = i + 1 < P.g.rows;
     const bool valid = j < P.g.columns;
     const bool has_right = j + 2 < P.g.columns;  // of the pair's second sample
-    const unsigned here = (static_cast<unsigned>(i) * P.g.pitch + j) * 4u;
+    const Offset here = (plane_row(i) * P.g.pitch + j) * 4u;
     const Pair rho = pair(P.rho), rest = pair(P.rest), two = pair(2.0f);
     auto across_or_0 = [&](Pair p) -> Pair { return pair(first(p), has_right ? second(p) : 0.0f); };
     auto down_or_0 = [&](Pair p) -> Pair { return has_down ? p : pair(0.0f); };
@@ -520,7 +535,7 @@ struct Walk {
     };
     auto left_of = [&](int q, int c, Pair p) -> Pair { return pair(own_row[exchange(q, c) + before], first(p)); };
     if constexpr (TGV) {
-      const Ball unit(P.radius0);
+      const Ball unit(radius0());
       Pair r11[C], r22[C], r12[C];
       Pair square = 0;
 #pragma unroll
@@ -529,10 +544,10 @@ struct Walk {
         const Pair u1 = above_at(2, c), u2 = above_at(3, c);
         const Pair exx = sub2(l1, across_or_0(k.nb1[c])), eyy = sub2(u2, down_or_0(k.nb2[c]));
         const Pair exy = mul2(pair(0.5f), add2(sub2(u1, down_or_0(k.nb1[c])), sub2(l2, across_or_0(k.nb2[c]))));
-        const Pair sigma = pair(P.sigma[c]);
-        r11[c] = fma2(sigma, exx, k.r11[c]);
-        r22[c] = fma2(sigma, eyy, k.r22[c]);
-        r12[c] = fma2(sigma, exy, k.r12[c]);
+        const Pair sigma_c = pair(sigma(c));
+        r11[c] = fma2(sigma_c, exx, k.r11[c]);
+        r22[c] = fma2(sigma_c, eyy, k.r22[c]);
+        r12[c] = fma2(sigma_c, exy, k.r12[c]);
         const Pair own = fma2(two, mul2(r12[c], r12[c]), fma2(r11[c], r11[c], mul2(r22[c], r22[c])));
         square = !COUPLED || c == 0 ? own : add2(square, own);
         if constexpr (!COUPLED) {
@@ -570,7 +585,7 @@ struct Walk {
       const Pair dy = sub2(down_or_0(k.pn2[c]), above_at(1, c));
       const Pair dx = sub2(across_or_0(k.pn1[c]), left_of(0, c, k.pn1[c]));
       float* to = c == 0 ? luma : chroma + (c - 1) * 8 * CR * WIDTH;
-      *reinterpret_cast<Pair*>(to + 32 * part + across) = fma2(pair(P.tau[c]), add2(dy, dx), k.xn[c]);
+      *reinterpret_cast<Pair*>(to + 32 * part + across) = fma2(pair(tau(c)), add2(dy, dx), k.xn[c]);
     }
   }
 
@@ -671,15 +686,15 @@ struct Walk {
         const float r11 = S(a, 5), r22 = S(a, 6), r12 = S(a, 7), w1 = S(a, 3), w2 = S(a, 4);
         const float d1 = __fadd_rn(__fsub_rn(S(a + 1, 5), r11), lower ? __fsub_rn(S(d, 7), r12) : 0.0f);
         const float d2 = __fadd_rn(__fsub_rn(S(a + 1, 7), r12), lower ? __fsub_rn(S(d, 6), r22) : 0.0f);
-        nb1 = fmaf(fmaf(P.tau[c], __fadd_rn(S(a, 1), d1), w1), -2.0f, w1);
-        nb2 = fmaf(fmaf(P.tau[c], __fadd_rn(S(a, 2), d2), w2), -2.0f, w2);
+        nb1 = fmaf(fmaf(tau(c), __fadd_rn(S(a, 1), d1), w1), -2.0f, w1);
+        nb2 = fmaf(fmaf(tau(c), __fadd_rn(S(a, 2), d2), w2), -2.0f, w2);
       }
       const float bar = fmaf(X(a), -2.0f, S(a, 0));
       const float gx = __fsub_rn(bar, fmaf(X(a + 1), -2.0f, S(a + 1, 0)));
       const float gy = lower ? __fsub_rn(bar, fmaf(X(d), -2.0f, S(d, 0))) : 0.0f;
       old1 = S(a, 1);
-      step1 = fmaf(P.sigma[c], TGV ? __fadd_rn(gx, nb1) : gx, old1);
-      step2 = fmaf(P.sigma[c], TGV ? __fadd_rn(gy, nb2) : gy, S(a, 2));
+      step1 = fmaf(sigma(c), TGV ? __fadd_rn(gx, nb1) : gx, old1);
+      step2 = fmaf(sigma(c), TGV ? __fadd_rn(gy, nb2) : gy, S(a, 2));
       const float s = SQUARE_2 ? step2 : step1, t = SQUARE_2 ? step1 : step2;
       square = fmaf(s, s, __fmul_rn(t, t));
     }
@@ -693,7 +708,7 @@ struct Walk {
       square = total;
     }
     if (mine) {
-      const float q1 = __fmul_rn(step1, ball(square, Ball(P.radius)));
+      const float q1 = __fmul_rn(step1, ball(square, Ball(radius())));
       float* to = shared + W::EXCHANGE + (row < kChunk - 1 ? row : row + (k & 1)) * W::ROW - 1 - (k & 1);
       to[exchange(0, c)] =
           REST_FIRST ? fmaf(P.rest, old1, __fmul_rn(P.rho, q1)) : fmaf(P.rho, q1, __fmul_rn(P.rest, old1));
@@ -719,7 +734,11 @@ struct Walk {
         if (lane == 0) {
           const int s = issued % kSlots;
           barrier_expect(&bars.full[s], (W::F + 1) * C * W::PLANE * 4);
-          load_box(shared + s * W::SLOT, map, &bars.full[s], x0 - kHalo, i0 - 2 + 2 * issued, 0);
+          if constexpr (UNROLLED) {
+            load_fields(shared + s * W::SLOT, map, &bars.full[s], x0 - kHalo, i0 - 2 + 2 * issued, image);
+          } else {
+            load_box(shared + s * W::SLOT, map, &bars.full[s], x0 - kHalo, i0 - 2 + 2 * issued, 0);
+          }
         }
       }
     };
