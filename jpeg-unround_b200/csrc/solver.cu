@@ -43,9 +43,12 @@ int samples_kernels() {
   return 0;
 }
 
-// Iterations that keep nothing are launched kGraphIterations at a time as one CUDA graph
-// (Impl::group; an even count, so that a group leaves the state's parity as it found it);
-// UNROUND_B200_GRAPHS=0 launches every iteration's kernels one by one.
+// Iterations that keep nothing and take several launches (the split kernels) are launched
+// kGraphIterations at a time as one CUDA graph (Impl::group; an even count, so that a group leaves
+// the state's parity as it found it); UNROUND_B200_GRAPHS=0 launches every iteration's kernels one
+// by one. The walk goes launch by launch: one costs the host 2.3 us, less than the shortest walk
+// (4.4 us) takes the device, while making a graph costs a call 0.2-0.3 ms (a 160x120 picture's solve
+// 1.04 -> 0.84 ms without, 512x512 2.2 -> 1.9; photographs and larger alike either way).
 constexpr std::uint64_t kGraphIterations = 8;
 
 bool group_graphs() {
@@ -125,9 +128,8 @@ struct Solver::Impl {
   // group after both launches have run eagerly (which sets up their launchers), made again for
   // the other parity.
   cudaGraphExec_t group_exec = nullptr;
-  int group_parity = -1, group_xt = -1;
+  int group_parity = -1;
   bool plain_dual = false, plain_primal = false;  // a dual(false) and a primal(false) have run
-  bool plain_fused = false;                       // a fused() has run
 
   Impl(const Frame& f, cudaStream_t s) : frame(f), stream(s) {}
 
@@ -619,26 +621,23 @@ struct Solver::Impl {
   // launches depend on the iteration only through the parity of the state, which an even count
   // of iterations leaves as it found it.
   bool group() {
-    const bool ready = fusable ? walks && plain_fused : plain_dual && plain_primal;
-    if (!ready || samples != nullptr || error != cudaSuccess || !group_graphs()) return false;
-    if (group_exec == nullptr || group_parity != current || group_xt != xt_id) {
+    if (!plain_dual || !plain_primal || fusable || samples != nullptr || error != cudaSuccess || !group_graphs()) {
+      return false;
+    }
+    if (group_exec == nullptr || group_parity != current) {
       if (group_exec != nullptr) {
         cudaGraphExecDestroy(group_exec);
         group_exec = nullptr;
       }
-      const int parity = current, buffer = xt_id;
+      const int parity = current;
       cudaGraph_t graph = nullptr;
       if (cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
         cudaGetLastError();
         return false;
       }
       for (std::uint64_t k = 0; k < kGraphIterations; ++k) {
-        if (fusable) {
-          fused();
-        } else {
-          dual(false);
-          primal(false);
-        }
+        dual(false);
+        primal(false);
       }
       const cudaError_t ended = cudaStreamEndCapture(stream, &graph);
       if (error == cudaSuccess) error = ended;
@@ -646,14 +645,12 @@ struct Solver::Impl {
       if (graph != nullptr) cudaGraphDestroy(graph);
       if (error != cudaSuccess) return false;
       group_parity = parity;
-      group_xt = buffer;
     }
     error = cudaGraphLaunch(group_exec, stream);
     return error == cudaSuccess;
   }
 
   void fused(WalkKeep keep = WalkKeep::nothing) {
-    plain_fused = plain_fused || keep == WalkKeep::nothing;
     record_xt = xt;
     if (samples != nullptr && samples_layout == 2) {
       SamplesStep q;

@@ -36,10 +36,10 @@
 // begins: of 56 looks at the ring, 55 need no wait. A launch's CTAs start on the places that the one
 // before leaves (programmatic dependent launch) and wait for its end with their barriers and
 // factors ready: 1-5 us of an iteration (160x120 5.2 -> 4.4, 2048^2 of three channels 174 -> 168).
-// Measured, an iteration as graphs of eight, before (two or three launches) and after: TV grey
-// 160x120 12.6 -> 4.4 us, 512^2 13.3 -> 5.4; TGV grey 512^2 18.4 -> 8.5, 2048^2 74 -> 66; TGV 4:2:0
-// 768x512 36.7 -> 19.2, 2048^2 200 -> 168; TV 4:2:0 1919x1083 63.2 -> 44.8, 2048^2 101 (two CTAs an
-// SM, a barrier for each tile) -> 85.
+// Measured, an iteration before (two or three launches, in graphs of eight) and after: TV grey
+// 160x120 12.6 -> 4.4 us, 512^2 13.3 -> 4.8; TGV grey 512^2 18.4 -> 8.6, 2048^2 74 -> 65; TGV 4:2:0
+// 768x512 36.7 -> 18.6, 2048^2 200 -> 167; TV 4:2:0 1919x1083 63.2 -> 44.1, 2048^2 101 (two CTAs an
+// SM, a barrier for each tile) -> 84.
 #pragma once
 
 #include <algorithm>
@@ -899,7 +899,14 @@ cudaError_t launch_one(const CUtensorMap& map, const IterationParams& p, cudaStr
     resident[device & 63].store(ctas);
   }
   IterationParams q = p;
-  q.strip_rows = walk_rows(p.dual.g, ctas, W::WIDTH, 8 * CR);
+  // The last picture's strip height: the same for all of a solve's launches.
+  thread_local struct {
+    int rows = 0, columns = 0, ctas = 0, height = 0;
+  } last;
+  if (last.rows != p.dual.g.rows || last.columns != p.dual.g.columns || last.ctas != ctas) {
+    last = {p.dual.g.rows, p.dual.g.columns, ctas, walk_rows(p.dual.g, ctas, W::WIDTH, 8 * CR)};
+  }
+  q.strip_rows = last.height;
   const dim3 grid((p.dual.g.columns + W::WIDTH - 1) / W::WIDTH, (p.dual.g.rows + q.strip_rows - 1) / q.strip_rows);
   if (partials != nullptr) *partials = static_cast<int>(grid.x * grid.y) * (C == 1 ? 2 : 1);
   cudaLaunchConfig_t config = {};
