@@ -231,42 +231,48 @@ __global__ void __launch_bounds__(256) primal_kernel(Problem q, Planes s, float*
 // `b` and the adjoint of x~_k into `xt_bar`. Gradients: [0] alpha0, [1] alpha1, [2] tau,
 // [3] sigma, each [image].
 //
-// The dual step's adjoint is one kernel over tiles of 16 rows x 32 columns. A tile's CTA loads,
+// The dual step's adjoint is one kernel over tiles of 14 rows x 32 columns. A tile's CTA loads,
 // by two 4D bulk-tensor copies, the 9 planes of s_{k-1} and x~_k and the 9 of the adjoint with
 // halos (2 rows above and 2 below, 4 columns each side: whole 16-byte words), and then in shared
 // memory: w~ over the tile and a ring of 2 (1), the adjoints of the projections' points q and s
 // over the tile and a ring of 1 (2), the adjoint of w~ over the tile and the ring's left column
 // and upper row (3), and the tile's adjoints (4). A halo's values are recomputed by each tile
 // that needs them; the gradients count the tile's own pixels only.
-constexpr int kAdjointRows = 16;                 // a tile's rows
+//
+// What bounds it: latency. Shared memory's loads are half of its time, its instructions the like and
+// HBM 60%, but each CTA goes through the copies' arrival and four phases between barriers one after
+// another, and only the other CTAs of its SM fill the gaps. So what (2) and (3) make is put where the
+// state was (nothing else is kept but w-), and 14 rows are the most with which four CTAs fit (56 KB
+// each). 16 pictures of 512 x 512: with arrays of their own and three CTAs of 16 rows 119 us, in
+// place with those 114, with four of 14 rows 106; of 12 rows 116, 10 rows and five CTAs 112. More
+// threads a CTA, or pairs of columns by the packed operations, were slower in every tile.
+constexpr int kAdjointRows = 14;                 // a tile's rows
+constexpr int kAdjointCtas = 4;                  // an SM's
 constexpr int kAdjointSpan = 40;                 // columns of a box: 4 + 32 + 4
-constexpr int kStateRows = kAdjointRows + 4;     // s_{k-1}, x~_k: rows i0 - 2 .. i0 + 17
-constexpr int kBarRows = kAdjointRows + 3;       // the adjoint: rows i0 - 1 .. i0 + 17
+constexpr int kStateRows = kAdjointRows + 4;     // s_{k-1}, x~_k: rows i0 - 2 .. i0 + 15
+constexpr int kBarRows = kAdjointRows + 3;       // the adjoint: rows i0 - 1 .. i0 + 15
 constexpr int kFields = 9;
 constexpr int kTildeRows = kAdjointRows + 3, kTildeColumns = 36;  // (1): rows i0 - 2 .., columns j0 - 2 ..
 constexpr int kPointRows = kAdjointRows + 2, kPointColumns = 34;  // (2): rows i0 - 1 .., columns j0 - 1 ..
 constexpr int kBackRows = kAdjointRows + 1, kBackColumns = 33;    // (3): rows i0 - 1 .., columns j0 - 1 ..
-constexpr int kStateFloats = kFields * kStateRows * kAdjointSpan;
+constexpr int kStateBox = kFields * kStateRows * kAdjointSpan;
+constexpr int kStateFloats = (kStateBox + 31) / 32 * 32;  // the adjoint's box starts 128-byte aligned
 constexpr int kBarFloats = kFields * kBarRows * kAdjointSpan;
-// (1), (2) and (3) are kept in rows of kAdjointSpan, as the boxes are, and walked as rows x
+// w- is kept in rows of kAdjointSpan, as the boxes are, and (1), (2) and (3) walked as rows x
 // kAdjointSpan points (the columns past each one's width idle): a warp's 32 points are 32
 // consecutive words of every array it reads or writes, across row ends too.
 constexpr int kTildeFloats = 2 * kTildeRows * kAdjointSpan;
-constexpr int kPointFloats = 5 * kPointRows * kAdjointSpan;
-static_assert(2 * kBackRows * kAdjointSpan <= kTildeFloats, "(3) reuses the space of (1)");
-static_assert(kStateFloats % 32 == 0, "the adjoint's box starts 128-byte aligned");
 constexpr std::size_t kAdjointShared =
-    static_cast<std::size_t>(kStateFloats + kBarFloats + kTildeFloats + kPointFloats) * sizeof(float);
+    static_cast<std::size_t>(kStateFloats + kBarFloats + kTildeFloats) * sizeof(float);
 
-__global__ void __launch_bounds__(256) dual_adjoint_kernel(const __grid_constant__ CUtensorMap state_map,
-                                                           const __grid_constant__ CUtensorMap bar_map, Problem q,
-                                                           Planes b, float* xt_bar, double* grads) {
+__global__ void __launch_bounds__(256, kAdjointCtas)
+    dual_adjoint_kernel(const __grid_constant__ CUtensorMap state_map, const __grid_constant__ CUtensorMap bar_map,
+                        Problem q, Planes b, float* xt_bar, double* grads) {
   extern __shared__ __align__(128) float shared[];
   __shared__ __align__(8) std::uint64_t loaded[2];  // [0] s_{k-1} and x~_k, [1] the adjoint
   float* const S = shared;                       // [field][row][column], row i0 - 2 + r, column j0 - 4 + c
   float* const A = S + kStateFloats;             // [field][row][column], row i0 - 1 + r, column j0 - 4 + c
-  float* const T = A + kBarFloats;               // (1) w~, then (3) the adjoint of w~
-  float* const L = T + kTildeFloats;             // (2) q^1, q^2, s^11, s^22, s^12
+  float* const T = A + kBarFloats;               // (1) w-
   const int tid = threadIdx.y * 32 + threadIdx.x;
   const int z = blockIdx.z, i0 = blockIdx.y * kAdjointRows, j0 = blockIdx.x * 32;
   const int H = q.rows, W = q.columns;
@@ -282,7 +288,7 @@ __global__ void __launch_bounds__(256) dual_adjoint_kernel(const __grid_constant
   // still on its way.
   if (tid == 0) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_address(&loaded[0])),
-                 "r"(static_cast<unsigned>(kStateFloats * sizeof(float)))
+                 "r"(static_cast<unsigned>(kStateBox * sizeof(float)))
                  : "memory");
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_address(&loaded[1])),
                  "r"(static_cast<unsigned>(kBarFloats * sizeof(float)))
@@ -304,16 +310,18 @@ __global__ void __launch_bounds__(256) dual_adjoint_kernel(const __grid_constant
     give_up();
     return;
   }
-  auto s_at = [&](int f, int i, int j) -> float { return S[(f * kStateRows + i - i0 + 2) * kAdjointSpan + j - j0 + 4]; };
+  auto s_at = [&](int f, int i, int j) -> float& { return S[(f * kStateRows + i - i0 + 2) * kAdjointSpan + j - j0 + 4]; };
   auto a_at = [&](int f, int i, int j) -> float { return A[(f * kBarRows + i - i0 + 1) * kAdjointSpan + j - j0 + 4]; };
   auto t_at = [&](int f, int i, int j) -> float& { return T[(f * kTildeRows + i - i0 + 2) * kAdjointSpan + j - j0 + 2]; };
-  auto l_at = [&](int f, int i, int j) -> float& { return L[(f * kPointRows + i - i0 + 1) * kAdjointSpan + j - j0 + 1]; };
-  auto tb_at = [&](int f, int i, int j) -> float& { return T[(f * kBackRows + i - i0 + 1) * kAdjointSpan + j - j0 + 1]; };
   enum { X = 0, P1, P2, W1, W2, R11, R22, R12, EXTRA };  // EXTRA: x~ in S, v^ in A
+  // What (1), (2) and (3) make at a pixel goes where they alone still read there: p + div2 r over w,
+  // the adjoints of q and s over p and r, that of w~ over x and x~.
+  auto l_at = [&](int f, int i, int j) -> float& { return s_at(f < 2 ? P1 + f : R11 + f - 2, i, j); };
+  auto tb_at = [&](int f, int i, int j) -> float& { return s_at(f == 0 ? X : EXTRA, i, j); };
   float g_alpha0 = 0.0f, g_alpha1 = 0.0f, g_sigma = 0.0f, g_tau = 0.0f;
-  // A tile whose halos lie inside the picture (rows i0 - 2 .. i0 + 17, columns j0 - 2 .. j0 + 34)
+  // A tile whose halos lie inside the picture (rows i0 - 2 .. i0 + 15, columns j0 - 2 .. j0 + 34)
   // passes every bounds test below: IN states that, and the tests fold away.
-  const bool interior = i0 >= 2 && j0 >= 2 && i0 + 17 < H && j0 + 34 < W;
+  const bool interior = i0 >= 2 && j0 >= 2 && i0 + kAdjointRows + 1 < H && j0 + 34 < W;
   bool failed = false;  // the same in every thread: set after a CTA-wide vote
   auto tile = [&](auto kind) {
     constexpr bool IN = decltype(kind)::value;
@@ -329,9 +337,12 @@ __global__ void __launch_bounds__(256) dual_adjoint_kernel(const __grid_constant
       d2 = d2 + (IN || i + 1 < H ? s_at(R22, i + 1, j) - r22 : 0.0f);
       // Kept as w- = 2 w~ - w, the only form (2) reads.
       const float w1 = s_at(W1, i, j), w2 = s_at(W2, i, j);
-      const float tilde1 = w1 + tau * (s_at(P1, i, j) + d1), tilde2 = w2 + tau * (s_at(P2, i, j) + d2);
+      const float step1 = s_at(P1, i, j) + d1, step2 = s_at(P2, i, j) + d2;
+      const float tilde1 = w1 + tau * step1, tilde2 = w2 + tau * step2;
       t_at(0, i, j) = 2.0f * tilde1 - w1;
       t_at(1, i, j) = 2.0f * tilde2 - w2;
+      s_at(W1, i, j) = step1;
+      s_at(W2, i, j) = step2;
     }
     const bool adjoint_ready = barrier_wait(&loaded[1], 0);
     if (__syncthreads_or(!adjoint_ready)) {
@@ -465,12 +476,7 @@ __global__ void __launch_bounds__(256) dual_adjoint_kernel(const __grid_constant
       b.r22[k] = rest * a_at(R22, i, j) + l_at(3, i, j) + div22;
       b.r12[k] = rest * a_at(R12, i, j) + l_at(4, i, j) + div12;
       // d/dtau of w~ = p + div2 r.
-      const float r11 = s_at(R11, i, j), r22 = s_at(R22, i, j), r12 = s_at(R12, i, j);
-      float d1 = right ? s_at(R11, i, j + 1) - r11 : 0.0f;
-      float d2 = right ? s_at(R12, i, j + 1) - r12 : 0.0f;
-      d1 = d1 + (down ? s_at(R12, i + 1, j) - r12 : 0.0f);
-      d2 = d2 + (down ? s_at(R22, i + 1, j) - r22 : 0.0f);
-      g_tau += tb1 * (s_at(P1, i, j) + d1) + tb2 * (s_at(P2, i, j) + d2);
+      g_tau += tb1 * s_at(W1, i, j) + tb2 * s_at(W2, i, j);
       // The adjoint of x- : grad^T (sigma q^) = -div (sigma q^).
       const float div = (right ? l_at(0, i, j) : 0.0f) - (IN || j > 0 ? l_at(0, i, j - 1) : 0.0f) +
                         (down ? l_at(1, i, j) : 0.0f) - (IN || i > 0 ? l_at(1, i - 1, j) : 0.0f);
