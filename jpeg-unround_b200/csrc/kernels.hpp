@@ -508,6 +508,10 @@ struct SamplesStep {
 };
 cudaError_t launch_dual_samples(const CUtensorMap& state, const CUtensorMap& tilde, const DualParams& p,
                                 const SamplesStep& q, bool tgv, bool coupled, cudaStream_t stream);
+// The same as a walk (walk_samples.cu; 1 or 3 channels, walk_takes, maps as make_walk_map makes them, x~
+// behind the state it is made from): the default.
+cudaError_t launch_walk_samples(const CUtensorMap& map, const DualParams& dual, const SamplesStep& samples, bool tgv,
+                                bool coupled, cudaStream_t stream);
 cudaError_t launch_samples_iteration(const CUtensorMap& state, const CUtensorMap& tilde,
                                      const SamplesIterationParams& p, bool tgv, bool coupled, cudaStream_t stream);
 

@@ -32,15 +32,21 @@ Kernels chosen_kernels() {
   return Kernels::walk;
 }
 
-// How pictures of rounded samples iterate: 0 two launches (the dual sweep, then the primal
-// kernel: the default, the fastest measured); 1 the fused sweep of iteration.cu
-// (UNROUND_B200_KERNELS=fused); 2 the dual sweep with the primal step in it (=sweep).
+// How pictures of rounded samples iterate: 3 the walk of walk_samples.cu (the default from
+// kSamplesWalk samples on); 0 two launches (the dual sweep, then the primal kernel:
+// UNROUND_B200_KERNELS=split, and what the walk does not take); 1 the fused sweep of iteration.cu
+// (=fused); 2 the dual sweep with the primal step in it (=sweep). Smaller pictures than kSamplesWalk
+// keep the two launches that measure_samples tells of them (64x64 of three channels: 13-21 us an
+// iteration; the walk, of 128x128, takes 4.5).
+constexpr std::size_t kSamplesWalk = 1 << 15;
+
 int samples_kernels() {
   const char* value = std::getenv("UNROUND_B200_KERNELS");
-  if (value == nullptr) return 0;
+  if (value == nullptr) return 3;
+  if (std::strcmp(value, "split") == 0) return 0;
   if (std::strcmp(value, "fused") == 0) return 1;
   if (std::strcmp(value, "sweep") == 0) return 2;
-  return 0;
+  return 3;
 }
 
 // Iterations that keep nothing and take several launches (the split kernels) are launched
@@ -104,6 +110,8 @@ struct Solver::Impl {
   const float* record_xt = nullptr;  // x~ of the last dual step: the tilde point's, for its record
   bool fusable = false;
   bool walks = false;  // fusable, by the walk of walk.cuh
+  // Whether a walk can keep a record's values (of pictures of samples none does).
+  bool walk_keeps() const { return walks && samples == nullptr; }
   int cell_rows = 1, cell_columns = 1;
   CUtensorMap iteration_state_maps[2];
   CUtensorMap iteration_tilde_maps[2];
@@ -265,9 +273,10 @@ struct Solver::Impl {
     const Kernels kernels = chosen_kernels();
     const bool whole = solving && samples == nullptr && kernels != Kernels::split &&
                        iteration_takes(g, components.data(), static_cast<int>(components.size()));
-    walks = whole && kernels == Kernels::walk && walk_takes(g);
-    fusable = samples != nullptr ? solving && samples_layout != 0 && samples_iteration_takes(g)
-                                 : walks || (whole && kernels == Kernels::fused);
+    const bool swept_samples = samples != nullptr && solving && samples_layout != 0 && samples_iteration_takes(g);
+    const bool large = static_cast<std::size_t>(g.channels) * g.rows * g.columns >= kSamplesWalk;
+    walks = ((whole && kernels == Kernels::walk) || (swept_samples && samples_layout == 3 && large)) && walk_takes(g);
+    fusable = walks || (swept_samples && samples_layout != 3) || (whole && kernels == Kernels::fused);
     for (int s = 0; s < 2; ++s) state[s] = fields(with_tgv, walks ? &xts[s] : nullptr);
     tilde = fields(with_tgv);
     if (!walks) xts[0] = allocate<float>(n);
@@ -652,7 +661,7 @@ struct Solver::Impl {
 
   void fused(WalkKeep keep = WalkKeep::nothing) {
     record_xt = xt;
-    if (samples != nullptr && samples_layout == 2) {
+    if (samples != nullptr && samples_layout != 1) {
       SamplesStep q;
       q.levels = s_levels;
       q.ends = s_ends;
@@ -661,8 +670,9 @@ struct Solver::Impl {
       q.r = static_cast<float>(1.0 / (1.0 + t));
       q.next = xts[1 - xt_id];
       if (error == cudaSuccess) {
-        error = launch_dual_samples(state_maps[current], tilde_maps[xt_id], dual_params(), q, tgv, plan.coupled,
-                                    stream);
+        error = walks ? launch_walk_samples(iteration_state_maps[current], dual_params(), q, tgv, plan.coupled, stream)
+                      : launch_dual_samples(state_maps[current], tilde_maps[xt_id], dual_params(), q, tgv,
+                                            plan.coupled, stream);
       }
       current = 1 - current;
       xt_id = 1 - xt_id;
@@ -1163,7 +1173,7 @@ bool Solver::run(std::uint64_t first, const Observer& observer, Outcome& out, Fa
   auto take = [&](std::uint64_t iteration) -> bool {
     m.enqueue_record(iteration);
     pending = true;
-    return m.walks && !observer && !recorded(iteration + 1) ? false : settle();
+    return m.walk_keeps() && !observer && !recorded(iteration + 1) ? false : settle();
   };
   auto none_recorded = [&](std::uint64_t from, std::uint64_t to) {
     for (std::uint64_t n = from; n <= to; ++n) {
@@ -1192,7 +1202,7 @@ bool Solver::run(std::uint64_t first, const Observer& observer, Outcome& out, Fa
     // anything (no record after the dual step, none of the next iterate), or by the walk when one
     // of them does.
     if (m.fusable && next < most && !(recorded(next) && recorded(next + 1)) &&
-        (m.walks || (!recorded(next) && !recorded(next + 1)))) {
+        (m.walk_keeps() || (!recorded(next) && !recorded(next + 1)))) {
       m.fused(recorded(next) ? WalkKeep::duals : recorded(next + 1) ? WalkKeep::primal : WalkKeep::nothing);
       iteration = next;
       if (recorded(iteration)) stopped = take(iteration);

@@ -380,7 +380,9 @@ __device__ __noinline__ void general_row(float (&coef)[8], int4 levels, int m, b
   }
 }
 
-template <bool TGV, int C, bool COUPLED, int CR, int CC, int KEEP, bool UNROLLED = false>
+// RAGGED: a canvas that is not whole blocks (pictures of samples): a strip's last chunk may reach past
+// the last row, and the last pair of an odd number of columns past the last column.
+template <bool TGV, int C, bool COUPLED, int CR, int CC, int KEEP, bool UNROLLED = false, bool RAGGED = false>
 struct Walk {
   using W = WalkLayout<TGV, C, CR>;
   static constexpr int L = W::L, SPAN = W::SPAN, WIDTH = W::WIDTH, XS = WIDTH + 4;
@@ -427,12 +429,15 @@ struct Walk {
                                              float* to) const {
     const DualParams& P = Q.dual;
     const int o = kHalo + 32 * part + across, j = x0 + 32 * part + across;
-    const bool valid = j < P.g.columns;  // the pair (the columns are even)
+    const bool valid = j < P.g.columns && (!RAGGED || i < P.g.rows);  // the pair, or its first sample
+    const bool alone = RAGGED && j + 1 >= P.g.columns;               // the second past the last column
     const int next = j + 2 < P.g.columns ? o + 2 : o + 1;
     const Offset here = (plane_row(FIRST ? 0 : i) * P.g.pitch + j) * 4u;
     const Pair rho = pair(P.rho), rest = pair(P.rest), minus_two = pair(-2.0f);
     auto own_at = [&](int offset) -> Pair { return *reinterpret_cast<const Pair*>(own + offset + o); };
-    auto right_of = [&](int offset, Pair p) -> Pair { return pair(second(p), own[offset + next]); };
+    auto right_of = [&](int offset, Pair p) -> Pair {
+      return pair(alone ? first(p) : second(p), own[offset + next]);
+    };
     auto down_at = [&](int offset) -> Pair { return *reinterpret_cast<const Pair*>(down + offset + o); };
     auto put = [&](float* base, int c, Pair p) {
       if (!FIRST && valid) *reinterpret_cast<Pair*>(reinterpret_cast<char*>(base + c * P.g.plane) + here) = p;
@@ -446,7 +451,7 @@ struct Walk {
       const Pair bar = fma2(xt, minus_two, x);
       const float right = fmaf(own[tilde(c) + next], -2.0f, own[at(0, c) + next]);
       const Pair below = fma2(down_at(tilde(c)), minus_two, down_at(at(0, c)));
-      const Pair gx = sub2(bar, pair(second(bar), right));
+      const Pair gx = sub2(bar, pair(alone ? first(bar) : second(bar), right));
       const Pair gy = sub2(bar, below);
       k.xn[c] = fma2(rho, xt, mul2(rest, x));
       put(P.out.x, c, k.xn[c]);
@@ -521,11 +526,14 @@ struct Walk {
     const DualParams& P = Q.dual;
     const int j = x0 + 32 * part + across;
     const bool has_down = i + 1 < P.g.rows;
-    const bool valid = j < P.g.columns;
+    const bool valid = j < P.g.columns && (!RAGGED || i < P.g.rows);
     const bool has_right = j + 2 < P.g.columns;  // of the pair's second sample
+    const bool alone = RAGGED && j + 1 >= P.g.columns;
     const Offset here = (plane_row(i) * P.g.pitch + j) * 4u;
     const Pair rho = pair(P.rho), rest = pair(P.rest), two = pair(2.0f);
-    auto across_or_0 = [&](Pair p) -> Pair { return pair(first(p), has_right ? second(p) : 0.0f); };
+    auto across_or_0 = [&](Pair p) -> Pair {
+      return pair(alone ? 0.0f : first(p), has_right ? second(p) : 0.0f);
+    };
     auto down_or_0 = [&](Pair p) -> Pair { return has_down ? p : pair(0.0f); };
     auto put = [&](float* base, int c, Pair p) {
       if (valid) *reinterpret_cast<Pair*>(reinterpret_cast<char*>(base + c * P.g.plane) + here) = p;
@@ -879,39 +887,39 @@ int walk_rows(const Geometry& g, int ctas, int width, int band) {
   return best;
 }
 
-template <bool TGV, int C, bool COUPLED, int CR, int CC, int KEEP>
-cudaError_t launch_one(const CUtensorMap& map, const IterationParams& p, cudaStream_t s, int* partials) {
-  using W = WalkLayout<TGV, C, CR>;
-  auto kernel = walk_kernel<TGV, C, COUPLED, CR, CC, KEEP>;
-  constexpr std::size_t bytes = W::FLOATS * sizeof(float);
+// A walk of a picture by `kernel` (`bytes` of shared memory, strips of `width` columns, heights of whole
+// bands) with the arguments `map` and `args`, whose strip height, in `step`, is set here. *grid: its CTAs.
+template <typename Args>
+cudaError_t launch_strips(void (*kernel)(CUtensorMap, Args), int threads, std::size_t bytes, int width, int band,
+                          const CUtensorMap& map, Args& args, IterationParams& step, std::atomic<int> (&resident)[64],
+                          cudaStream_t s, int* ctas_of_grid = nullptr) {
   // Once per device: the shared-memory size above 48 KB, and how many CTAs the device holds.
-  static std::atomic<int> resident[64] = {};
   int device = 0;
   cudaGetDevice(&device);
   int ctas = resident[device & 63].load();
   if (ctas == 0) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
     int per_sm = 0, sms = 0;
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, walk_threads<C>(), bytes);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, bytes);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     if (e != cudaSuccess) return e;
     ctas = std::max(1, per_sm * sms);
     resident[device & 63].store(ctas);
   }
-  IterationParams q = p;
+  const Geometry& g = step.dual.g;
   // The last picture's strip height: the same for all of a solve's launches.
   thread_local struct {
-    int rows = 0, columns = 0, ctas = 0, height = 0;
+    int rows = 0, columns = 0, ctas = 0, width = 0, band = 0, height = 0;
   } last;
-  if (last.rows != p.dual.g.rows || last.columns != p.dual.g.columns || last.ctas != ctas) {
-    last = {p.dual.g.rows, p.dual.g.columns, ctas, walk_rows(p.dual.g, ctas, W::WIDTH, 8 * CR)};
+  if (last.rows != g.rows || last.columns != g.columns || last.ctas != ctas || last.width != width || last.band != band) {
+    last = {g.rows, g.columns, ctas, width, band, walk_rows(g, ctas, width, band)};
   }
-  q.strip_rows = last.height;
-  const dim3 grid((p.dual.g.columns + W::WIDTH - 1) / W::WIDTH, (p.dual.g.rows + q.strip_rows - 1) / q.strip_rows);
-  if (partials != nullptr) *partials = static_cast<int>(grid.x * grid.y) * (C == 1 ? 2 : 1);
+  step.strip_rows = last.height;
+  const dim3 grid((g.columns + width - 1) / width, (g.rows + step.strip_rows - 1) / step.strip_rows);
+  if (ctas_of_grid != nullptr) *ctas_of_grid = static_cast<int>(grid.x * grid.y);
   cudaLaunchConfig_t config = {};
   config.gridDim = grid;
-  config.blockDim = dim3(walk_threads<C>());
+  config.blockDim = dim3(threads);
   config.dynamicSmemBytes = bytes;
   config.stream = s;
   cudaLaunchAttribute early;
@@ -919,7 +927,18 @@ cudaError_t launch_one(const CUtensorMap& map, const IterationParams& p, cudaStr
   early.val.programmaticStreamSerializationAllowed = 1;
   config.attrs = &early;
   config.numAttrs = 1;
-  return cudaLaunchKernelEx(&config, kernel, map, q);
+  return cudaLaunchKernelEx(&config, kernel, map, args);
+}
+
+template <bool TGV, int C, bool COUPLED, int CR, int CC, int KEEP>
+cudaError_t launch_one(const CUtensorMap& map, const IterationParams& p, cudaStream_t s, int* partials) {
+  using W = WalkLayout<TGV, C, CR>;
+  static std::atomic<int> resident[64] = {};
+  IterationParams q = p;
+  const cudaError_t e = launch_strips(walk_kernel<TGV, C, COUPLED, CR, CC, KEEP>, walk_threads<C>(),
+                                      W::FLOATS * sizeof(float), W::WIDTH, 8 * CR, map, q, q, resident, s, partials);
+  if (partials != nullptr && C == 1) *partials *= 2;
+  return e;
 }
 
 template <bool TGV, bool COUPLED, int KEEP>
