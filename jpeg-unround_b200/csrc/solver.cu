@@ -53,7 +53,7 @@ int samples_kernels() {
 // kGraphIterations at a time as one CUDA graph (Impl::group; an even count, so that a group leaves
 // the state's parity as it found it); UNROUND_B200_GRAPHS=0 launches every iteration's kernels one
 // by one. The walk goes launch by launch: one costs the host 2.3 us, less than the shortest walk
-// (4.4 us) takes the device, while making a graph costs a call 0.2-0.3 ms (a 160x120 picture's solve
+// (3.7 us) takes the device, while making a graph costs a call 0.2-0.3 ms (a 160x120 picture's solve
 // 1.04 -> 0.84 ms without, 512x512 2.2 -> 1.9; photographs and larger alike either way).
 constexpr std::uint64_t kGraphIterations = 8;
 

@@ -239,8 +239,8 @@ __global__ void __launch_bounds__(256) primal_kernel(Problem q, Planes s, float*
 // and upper row (3), and the tile's adjoints (4). A halo's values are recomputed by each tile
 // that needs them; the gradients count the tile's own pixels only.
 //
-// What bounds it: latency. Shared memory's loads are half of its time, its instructions the like and
-// HBM 60%, but each CTA goes through the copies' arrival and four phases between barriers one after
+// What bounds it: latency. Shared memory's accesses are half of its time, its instructions two thirds
+// and HBM 60%, but each CTA goes through the copies' arrival and four phases between barriers one after
 // another, and only the other CTAs of its SM fill the gaps. So what (2) and (3) make is put where the
 // state was (nothing else is kept but w-), and 14 rows are the most with which four CTAs fit (56 KB
 // each). 16 pictures of 512 x 512: with arrays of their own and three CTAs of 16 rows 119 us, in

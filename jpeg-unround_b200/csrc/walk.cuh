@@ -35,10 +35,13 @@
 // what is rarely run is not inlined: 4032x3024 TV 331 -> 261 us). Its rows are there when a chunk
 // begins: of 56 looks at the ring, 55 need no wait. A launch's CTAs start on the places that the one
 // before leaves (programmatic dependent launch) and wait for its end with their barriers and
-// factors ready: 1-5 us of an iteration (160x120 5.2 -> 4.4, 2048^2 of three channels 174 -> 168).
+// factors ready: 1-5 us of an iteration (160x120 5.2 -> 3.7, 2048^2 of three channels 174 -> 168).
+// They let the next launch's in only after their own wait. Let in at once, launches waited in chains,
+// as deep as small grids leave places, and with four solves on streams of their own the device
+// reported a failed launch.
 // Measured, an iteration before (two or three launches, in graphs of eight) and after: TV grey
-// 160x120 12.6 -> 4.4 us, 512^2 13.3 -> 4.8; TGV grey 512^2 18.4 -> 8.6, 2048^2 74 -> 65; TGV 4:2:0
-// 768x512 36.7 -> 18.6, 2048^2 200 -> 167; TV 4:2:0 1919x1083 63.2 -> 44.1, 2048^2 101 (two CTAs an
+// 160x120 12.6 -> 3.7 us, 512^2 13.3 -> 4.5; TGV grey 512^2 18.4 -> 8.4, 2048^2 74 -> 64; TGV 4:2:0
+// 768x512 36.7 -> 18.2, 2048^2 200 -> 167; TV 4:2:0 1919x1083 63.2 -> 43.9, 2048^2 101 (two CTAs an
 // SM, a barrier for each tile) -> 84.
 #pragma once
 
@@ -609,13 +612,13 @@ struct Walk {
     const int tries = static_cast<int>(min(P.ring_wait_limit, kWaitLimit));
     auto ready = [&](int n) { return wait_unless(&bars.full[n % kSlots], (n / kSlots) & 1, failed, tries); };
     // The row above the strip: its -w- and p2_n, as a chunk's row 7 before the first (0 above the
-    // canvas).
+    // canvas). Slot 0 is waited for there too: no slot is filled again, and no CTA leaves, before what
+    // was on its way to it has landed.
     bool good = true;
     if (warp == 0) {
       float* const to = row_of(kChunk - 1, 1);
+      good = __all_sync(kAll, ready(0) && ready(1));
       if (i0 > 0) {
-        good = ready(0) && ready(1);
-        good = __all_sync(kAll, good);
         if (good) {
           Kept kept[L];
 #pragma unroll
@@ -751,8 +754,11 @@ struct Walk {
       }
     };
     // Nothing of the state is read or written before the launch before this one is done: every other
-    // warp waits for rows that are copied from here on.
+    // warp waits for rows that are copied from here on. Only then may the next launch's CTAs take the
+    // places that this one's leave (to wait here, with what does not depend on it done): one launch
+    // waits at a time, never a chain of them.
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     issue_to(kSlots);
     if (!left_column(bars, failed, 0, lane)) return false;
     for (int k = 0; k < chunks; ++k) {
@@ -810,9 +816,6 @@ __global__ void __launch_bounds__(walk_threads<C>(), walk_ctas<TGV, C>())
   __shared__ WalkFactors factors[C];
   __shared__ int failed;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  // The next iteration's CTAs may take the places that this one's leave; they wait for its end
-  // (copy_warp) with what does not depend on it done.
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 #pragma unroll
   for (int c = 0; c < C; ++c) {
     const ProxFactors* all = Q.component[c].factors;

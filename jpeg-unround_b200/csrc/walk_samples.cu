@@ -28,7 +28,6 @@ __global__ void __launch_bounds__(walk_threads<C>(), walk_ctas<TGV, C>())
   __shared__ __align__(8) WalkBarriers bars;
   __shared__ int failed;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (tid == 0) {
     for (int s = 0; s < kSlots; ++s) barrier_init(&bars.full[s], 1);
     for (int s = 0; s < 2; ++s) {

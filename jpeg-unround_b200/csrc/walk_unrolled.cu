@@ -97,7 +97,6 @@ __global__ void __launch_bounds__(walk_threads<1>(), 3)
   __shared__ ClipTable table;
   __shared__ int failed;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, image = blockIdx.z;
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const float tau = __ldg(P.tau + image);
   for (int n = tid; n < 128; n += walk_threads<1>()) {
     const int k = n & 63;
