@@ -46,6 +46,9 @@ UNIT = "Mpx*iter/s"
 ALGORITHMIC_BYTES = 65.0
 # The dual kernel alone: x~, x, w(2), p(2), r(3) read and x, w, p, r written.
 DUAL_BYTES = 17 * 4.0
+# An iteration as one launch, the walk: x~ of the next iteration written beside, and the levels read
+# (4:2:0; one channel and samples read 2 B of levels a sample).
+WALK_BYTES, WALK_BYTES_2 = 18 * 4.0 + 1, 18 * 4.0 + 2
 
 
 def _rank() -> tuple[int, int, int]:
@@ -263,13 +266,20 @@ def _parity(decoded, theirs, image) -> dict:
             "inside_intervals": inside, "bar": {"rel_l2": 1e-4, "max_abs": 2e-3, "same_8bit": 0.999}}
 
 
-def _traffic() -> float | None:
-    """DRAM bytes per launch of the dual kernel at this workload, from the committed ncu summary."""
+def _traffic(timing) -> float | None:
+    """DRAM bytes per launch of the timed kernel at this workload, from the committed ncu summary."""
     path = ROOT / "profiles" / "traffic.json"
+    kernel = "walk" if timing.launches_per_iteration == 1 else "dual"
     try:
-        return float(json.loads(path.read_text())["dual_kernel_bytes_per_launch_4032x3024_420"])
+        return float(json.loads(path.read_text())[f"{kernel}_kernel_bytes_per_launch_4032x3024_420"])
     except (OSError, KeyError, ValueError):
         return None
+
+
+def _timed_kernel(timing, walk: str, walk_bytes: float, dual: str) -> tuple[str, float]:
+    """The kernel that dual_milliseconds times and its algorithmic bytes a sample: a walk where an
+    iteration is one launch, the dual sweep where it is several."""
+    return (walk, walk_bytes) if timing.launches_per_iteration == 1 else (dual, DUAL_BYTES)
 
 
 def _jpeg_file(seed: int) -> bytes:
@@ -586,9 +596,13 @@ def _samples_arm(args: argparse.Namespace, rank: int, world: int) -> None:
         d2h = call()
     e2e_seconds = max_over_ranks(time.perf_counter() - began)
     peak, peak_kind = _peaks()
-    dual = DUAL_BYTES * timing.samples / (timing.dual_milliseconds / 1e3) / 1e9
-    primal = SAMPLES_BYTES * timing.samples / (timing.primal_milliseconds / 1e3) / 1e9
-    iteration = (DUAL_BYTES + SAMPLES_BYTES) * timing.samples / (seconds / (args.steps * ITERATIONS)) / 1e9
+    kernel, kernel_bytes = _timed_kernel(timing, "walk_samples_kernel<tgv,3,coupled>", WALK_BYTES_2,
+                                         "dual_kernel<tgv,3,coupled>")
+    dual = kernel_bytes * timing.samples / (timing.dual_milliseconds / 1e3) / 1e9
+    # An iteration as one launch has no primal launch of its own to time.
+    split = timing.launches_per_iteration > 1
+    primal = SAMPLES_BYTES * timing.samples / (timing.primal_milliseconds / 1e3) / 1e9 if split else None
+    iteration = (DUAL_BYTES + SAMPLES_BYTES if split else kernel_bytes) * timing.samples / (seconds / (args.steps * ITERATIONS)) / 1e9
     if rank != 0:
         return
     line = {
@@ -600,11 +614,12 @@ def _samples_arm(args: argparse.Namespace, rank: int, world: int) -> None:
         "dtype": "f32", "data": "synthetic (the bench's colour picture, RGB, 8-bit levels)",
         "config": {"workload": "samples-rgb8-4032x3024", "iterations_per_step": ITERATIONS, "alpha1": 1.0,
                    "alpha0": 2.0, "samples": timing.samples, "l2": "state larger than L2, no flush"},
-        "roofline": {"bound": "hbm", "kernel": "dual_kernel<tgv,3,coupled>", "achieved": dual, "peak": peak,
+        "roofline": {"bound": "hbm", "kernel": kernel, "achieved": dual, "peak": peak,
                      "unit": "GB/s", "frac": dual / peak, "peak_kind": peak_kind,
-                     "algorithmic_bytes_per_sample": DUAL_BYTES, "dual_ms": timing.dual_milliseconds,
-                     "samples_primal_achieved": primal, "samples_primal_frac": primal / peak,
-                     "samples_primal_bytes_per_sample": SAMPLES_BYTES, "primal_ms": timing.primal_milliseconds,
+                     "algorithmic_bytes_per_sample": kernel_bytes, "dual_ms": timing.dual_milliseconds,
+                     "samples_primal_achieved": primal, "samples_primal_frac": primal / peak if split else None,
+                     "samples_primal_bytes_per_sample": SAMPLES_BYTES if split else None,
+                     "primal_ms": timing.primal_milliseconds if split else None,
                      "iteration_achieved": iteration, "iteration_frac": iteration / peak,
                      "one_launch": {mode: {"iteration_ms": t.milliseconds / t.iterations,
                                            "bytes_per_sample": SAMPLES_FUSED_BYTES,
@@ -751,6 +766,8 @@ def _large_arm(args: argparse.Namespace, rank: int, world: int) -> None:
     inside = bool(np.all((zeta >= lower) & (zeta <= upper)))
     history = decoded.result.history
     peak, peak_kind = _peaks()
+    kernel, kernel_bytes = _timed_kernel(timing, "walk_kernel<tgv,1>", WALK_BYTES_2, "dual_tma_kernel<tgv,1>")
+    achieved = kernel_bytes * timing.samples / (timing.dual_milliseconds / 1e3) / 1e9
     if rank != 0:
         return
     line = {
@@ -760,13 +777,13 @@ def _large_arm(args: argparse.Namespace, rank: int, world: int) -> None:
         "dtype": "f32", "data": "synthetic (seeded piecewise-smooth + noise sigma 2, table steps U{1..64})",
         "config": {"workload": f"tgv-grey-{args.side}-custom", "alpha1": 1.5, "alpha0": 3.0, "iterations": iterations,
                    "samples": timing.samples, "l2": f"state {17 * 4 * timing.samples / 1e9:.2f} GB"},
-        "roofline": {"bound": "hbm", "kernel": "dual_tma_kernel<tgv,1>", "achieved":
-                     DUAL_BYTES * timing.samples / (timing.dual_milliseconds / 1e3) / 1e9, "peak": peak,
-                     "unit": "GB/s", "peak_kind": peak_kind,
-                     "frac": DUAL_BYTES * timing.samples / (timing.dual_milliseconds / 1e3) / 1e9 / peak,
+        "roofline": {"bound": "hbm", "kernel": kernel, "achieved": achieved, "peak": peak,
+                     "unit": "GB/s", "peak_kind": peak_kind, "frac": achieved / peak,
+                     "algorithmic_bytes_per_sample": kernel_bytes,
                      "iteration_bytes_per_sample": 66.0,
                      "iteration_frac": 66.0 * timing.samples / (timing.milliseconds / iterations / 1e3) / 1e9 / peak,
-                     "dual_ms": timing.dual_milliseconds, "primal_ms": timing.primal_milliseconds},
+                     "dual_ms": timing.dual_milliseconds,
+                     "primal_ms": timing.primal_milliseconds if timing.launches_per_iteration > 1 else None},
         "gap_per_sample_every_50": [float(g) / timing.samples for g in history.gap],
         "record_iterations": [int(n) for n in history.iterations],
         "all_blocks_inside_intervals_fp64": inside, "blocks": int(zeta.size // 64),
@@ -780,17 +797,14 @@ def _large_arm(args: argparse.Namespace, rank: int, world: int) -> None:
 
 
 def _unrolled_forward_launches(iterations: int) -> int:
-    """The start, N primal steps and N - 1 dual steps."""
-    return 2 * iterations
+    """The start, the first primal step, and N - 1 walks (a dual step and the next primal step each)."""
+    return iterations + 1
 
 
 def _unrolled_backward_launches(iterations: int, every: int) -> int:
-    """Per segment of checkpoints K apart: the recomputed dual steps and primal steps, then the
-    dual steps' adjoints (N - 1) and the primal steps' adjoints (N)."""
-    launches = 0
-    for k0 in range(0, iterations, every):
-        k1 = min(k0 + every, iterations)
-        launches += (k1 - k0 - 1) + max(k1 - k0 - 2, 0) + (1 if k1 - k0 > 1 and k1 < iterations else 0)
+    """Per segment of checkpoints K apart the walks that recompute its states, then the dual steps'
+    adjoints (N - 1) and the primal steps' adjoints (N)."""
+    launches = sum(min(k0 + every, iterations) - k0 - 1 for k0 in range(0, iterations, every))
     return launches + (iterations - 1) + iterations
 
 
@@ -1024,10 +1038,12 @@ def main() -> None:
     peak, peak_kind = _peaks()
     copy = _copy_gbs()
     samples = timing.samples
-    dual_achieved = DUAL_BYTES * samples / (timing.dual_milliseconds / 1e3) / 1e9
+    kernel, kernel_bytes = _timed_kernel(timing, "walk_kernel<tgv,3,coupled,2,2>", WALK_BYTES,
+                                         "dual_kernel<tgv,3,coupled>")
+    dual_achieved = kernel_bytes * samples / (timing.dual_milliseconds / 1e3) / 1e9
     iteration_seconds = seconds / (args.steps * ITERATIONS)
     iteration_achieved = ALGORITHMIC_BYTES * samples / iteration_seconds / 1e9
-    traffic = _traffic()
+    traffic = _traffic(timing)
     if rank == 0:
         line = {
             "metric": METRIC, "value": value, "unit": UNIT,
@@ -1039,12 +1055,13 @@ def main() -> None:
             "config": {"workload": "tgv-colour-4032x3024-420", "iterations_per_step": ITERATIONS,
                        "alpha1": 1.0, "alpha0": 2.0, "samples": samples, "pixels": pixels,
                        "l2": "state larger than L2 (~3 GB), no flush", "parallelism": f"{world} independent images"},
-            "roofline": {"bound": "hbm", "kernel": "dual_kernel<tgv,3,coupled>", "achieved": dual_achieved,
+            "roofline": {"bound": "hbm", "kernel": kernel, "achieved": dual_achieved,
                          "peak": peak, "unit": "GB/s", "frac": dual_achieved / peak, "peak_kind": peak_kind,
-                         "traffic": traffic, "algorithmic_bytes_per_sample": DUAL_BYTES,
+                         "traffic": traffic, "algorithmic_bytes_per_sample": kernel_bytes,
                          "iteration_achieved": iteration_achieved, "iteration_frac": iteration_achieved / peak,
                          "iteration_bytes_per_sample": ALGORITHMIC_BYTES,
-                         "dual_ms": timing.dual_milliseconds, "primal_ms": timing.primal_milliseconds,
+                         "dual_ms": timing.dual_milliseconds,
+                         "primal_ms": timing.primal_milliseconds if timing.launches_per_iteration > 1 else None,
                          "copy_gbs_this_box": copy, "frac_of_copy_this_box": dual_achieved / copy,
                          "iteration_frac_of_copy_this_box": iteration_achieved / copy},
             "e2e": {"value": e2e, "unit": UNIT, "h2d_bytes_per_step": levels_bytes, "d2h_bytes_per_step": d2h},
