@@ -58,12 +58,13 @@ unround_status unround_b200_measure(const unround_input* input, const unround_se
  * picture a call): `count` inputs, each with its settings (tv or tgv, the same number of
  * iterations, --record-every 0), into `count` results, each freed by unround_result_free and
  * each the result unround_solve gives that picture alone to binary32 rounding. The iterations
- * but the last run for all pictures at once -- one launch per kernel class an iteration (the
- * dual sweep of each method and channel count, the primal step of each cell layout) over tables
- * of tiles of all pictures, two iterations captured in one CUDA graph launched for every pair.
- * `timing` (may be null) gets that part's device milliseconds (CUDA events), its iterations and
- * launches per iteration, and the samples and pixels of all pictures. On failure no result is
- * made. */
+ * but the last run for the smaller pictures at once -- one launch per kernel class an iteration
+ * (the dual sweep of each method and channel count, the primal step of each cell layout) over
+ * tables of tiles of all of them, two iterations captured in one CUDA graph launched for every
+ * pair -- and for the larger ones beside them, a launch a picture and iteration, a few pictures
+ * at a time. `timing` (may be null) gets the device milliseconds from the first of these launches
+ * to the end of the last (CUDA events), their iterations and launches per iteration, and the
+ * samples and pixels of all pictures. On failure no result is made. */
 typedef struct unround_b200_batch_timing {
   double milliseconds;
   uint64_t iterations;

@@ -175,6 +175,48 @@ int tune_dual(const DualClass& dual, const DualBatchImage* images_device, cudaSt
   return best_ms < 0.98f * model_ms ? best : model;
 }
 
+// Pictures of kWalkSamples samples or more that the walk takes iterate by launches of their own,
+// kLanes of them at a time on streams of their own, beside the batched launches of the others: a
+// walk moves 73 bytes a sample where the two batched steps move 85, and a picture's last iteration
+// and result come while the next ones iterate. A picture's share of an iteration, batched (12 alike)
+// and by walks in three lanes: TGV grey 384^2 3.60 and 3.27 us, 512^2 6.07 and 4.49, 1024^2 19.6
+// and 16.3; TGV 4:2:0 256^2 5.12 and 3.65, 512^2 15.0 and 13.2, 1024^2 51.3 and 47.7; TV 4:2:0
+// 256^2 3.02 and 2.59, 512^2 8.29 and 6.81, 1024^2 28.7 and 24.7. Below, the host's 2.3 us a launch
+// is what many small pictures would wait for (TV 4:2:0 192^2 2.39 and 2.55, 128^2 1.73 batched). TV
+// of one channel stays batched: its batched sweep fuses another product of a sum than the walk does.
+constexpr std::size_t kWalkSamples = 1 << 17;
+constexpr std::size_t kLanes = 3;
+
+bool wants_walk(const BatchEntry& e) {
+  const Frame& f = *e.frame;
+  return (e.plan.tgv || f.channels() > 1) && f.channels() * f.rows * f.columns >= kWalkSamples;
+}
+
+// The pictures that walk: a stream and the event of its iterations' end each.
+struct Walkers {
+  std::vector<std::size_t> pictures;
+  std::vector<cudaStream_t> streams;  // of every picture of the batch; null for one without
+  std::vector<cudaEvent_t> ends;
+  cudaError_t error = cudaSuccess;
+  explicit Walkers(const std::vector<BatchEntry>& entries) {
+    streams.resize(entries.size(), nullptr);
+    ends.resize(entries.size(), nullptr);
+    for (std::size_t n = 0; n < entries.size(); ++n) {
+      if (!wants_walk(entries[n])) continue;
+      if (error == cudaSuccess) error = cudaStreamCreateWithFlags(&streams[n], cudaStreamNonBlocking);
+      if (error == cudaSuccess) error = cudaEventCreate(&ends[n]);
+    }
+  }
+  ~Walkers() {
+    for (cudaStream_t s : streams) {
+      if (s != nullptr) cudaStreamDestroy(s);
+    }
+    for (cudaEvent_t e : ends) {
+      if (e != nullptr) cudaEventDestroy(e);
+    }
+  }
+};
+
 struct PrimalClass {
   int cell_rows = 1;
   int cell_columns = 1;
@@ -208,10 +250,17 @@ bool solve_batch(const std::vector<BatchEntry>& entries, cudaStream_t stream, st
   if (!check_batch(entries, failure)) return false;
   const std::uint64_t most = entries[0].plan.iterations;
   // Each picture's solver, started.
+  Walkers walkers(entries);
+  if (walkers.error != cudaSuccess) {
+    failure = {kInternal, "the batch's streams: " + describe(walkers.error)};
+    return false;
+  }
   std::vector<std::unique_ptr<Solver>> solvers;
-  for (const BatchEntry& e : entries) {
-    solvers.push_back(std::make_unique<Solver>(*e.frame, stream));
-    if (!solvers.back()->begin_batch(e.plan, failure)) return false;
+  for (std::size_t n = 0; n < entries.size(); ++n) {
+    const bool walking = walkers.streams[n] != nullptr;
+    solvers.push_back(std::make_unique<Solver>(*entries[n].frame, walking ? walkers.streams[n] : stream));
+    if (!solvers.back()->begin_batch(entries[n].plan, failure, walking)) return false;
+    if (walking && solvers.back()->walks()) walkers.pictures.push_back(n);
   }
   // The tables: each picture's entry, each component's, and per class the tiles and items.
   std::vector<DualBatchImage> images(entries.size());
@@ -230,6 +279,7 @@ bool solve_batch(const std::vector<BatchEntry>& entries, cudaStream_t stream, st
     const Plan& plan = entries[n].plan;
     timing.samples += static_cast<std::uint64_t>(g.channels) * g.rows * g.columns;
     timing.pixels += static_cast<std::uint64_t>(entries[n].frame->height) * entries[n].frame->width;
+    if (std::binary_search(walkers.pictures.begin(), walkers.pictures.end(), n)) continue;
     DualClass& dual = duals[{plan.tgv, g.channels, plan.coupled && g.channels > 1}];
     dual.tgv = plan.tgv;
     dual.channels = g.channels;
@@ -329,13 +379,13 @@ bool solve_batch(const std::vector<BatchEntry>& entries, cudaStream_t stream, st
   // the record and the result) runs on its own.
   const std::uint64_t batched = most > 0 ? most - 1 : 0;
   timing.iterations = batched;
-  timing.launches_per_iteration = primals.size() + duals.size();
+  timing.launches_per_iteration = primals.size() + duals.size() + walkers.pictures.size();
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   cudaEvent_t began = nullptr, ended = nullptr;
   if (error == cudaSuccess) error = cudaEventCreate(&began);
   if (error == cudaSuccess) error = cudaEventCreate(&ended);
-  if (batched > 2 && error == cudaSuccess) {
+  if (batched > 2 && !duals.empty() && error == cudaSuccess) {
     // Set up every launcher (shared memory, occupancy) before the capture: a launch of no work.
     for (auto& [key, primal] : primals) {
       if (error == cudaSuccess) {
@@ -368,27 +418,54 @@ bool solve_batch(const std::vector<BatchEntry>& entries, cudaStream_t stream, st
   // With an even count the last iteration (k = N - 1, of the pairs' first parity) is left.
   if (batched > 1 && (batched - 1) % 2 == 1) iteration(batched, stream);
   if (error == cudaSuccess) error = cudaEventRecord(ended, stream);
-  if (error == cudaSuccess) error = cudaEventSynchronize(ended);
-  float milliseconds = 0.0f;
-  if (error == cudaSuccess) error = cudaEventElapsedTime(&milliseconds, began, ended);
-  timing.milliseconds = milliseconds;
+  outcomes.clear();
+  outcomes.resize(entries.size());
+  bool good = true;
+  auto finish = [&](std::size_t n) {
+    if (!good || error != cudaSuccess || solvers[n]->finish_batch(batched, outcomes[n], failure)) return;
+    failure.message = "picture " + std::to_string(n) + ": " + failure.message;
+    good = false;
+  };
+  // The walking pictures, the largest first, so that the lanes end together: a picture's iterations
+  // follow those of the one kLanes before it, which is finished while they run; the batched ones are
+  // finished beside the last walks.
+  std::vector<std::size_t> order = walkers.pictures;
+  std::stable_sort(order.begin(), order.end(), [&](std::size_t x, std::size_t y) {
+    const Geometry &p = solvers[x]->geometry(), &q = solvers[y]->geometry();
+    return p.plane * p.channels > q.plane * q.channels;
+  });
+  for (std::size_t k = 0; k < order.size(); ++k) {
+    const std::size_t n = order[k];
+    if (good && error == cudaSuccess) {
+      error = cudaStreamWaitEvent(walkers.streams[n], k < kLanes ? began : walkers.ends[order[k - kLanes]], 0);
+      if (error == cudaSuccess) error = solvers[n]->walk(batched);
+      if (error == cudaSuccess) error = cudaEventRecord(walkers.ends[n], walkers.streams[n]);
+    }
+    if (k >= kLanes) finish(order[k - kLanes]);
+  }
+  for (std::size_t n = 0; n < entries.size(); ++n) {
+    if (std::find(order.begin(), order.end(), n) == order.end()) finish(n);
+  }
+  for (std::size_t k = order.size() - std::min(order.size(), kLanes); k < order.size(); ++k) finish(order[k]);
+  // From the first launch to the end of the last picture's iterations.
+  auto until = [&](cudaEvent_t end) {
+    float milliseconds = 0.0f;
+    if (good && error == cudaSuccess) error = cudaEventSynchronize(end);
+    if (good && error == cudaSuccess) error = cudaEventElapsedTime(&milliseconds, began, end);
+    timing.milliseconds = std::max(timing.milliseconds, static_cast<double>(milliseconds));
+  };
+  until(ended);
+  for (std::size_t n : order) until(walkers.ends[n]);
+  if (error != cudaSuccess) cudaStreamSynchronize(stream);
   if (exec != nullptr) cudaGraphExecDestroy(exec);
   if (graph != nullptr) cudaGraphDestroy(graph);
   if (began != nullptr) cudaEventDestroy(began);
   if (ended != nullptr) cudaEventDestroy(ended);
-  if (error != cudaSuccess) {
+  if (good && error != cudaSuccess) {
     failure = {kInternal, "the device failed in the batched iterations: " + describe(error)};
     return false;
   }
-  outcomes.clear();
-  outcomes.resize(entries.size());
-  for (std::size_t n = 0; n < entries.size(); ++n) {
-    if (!solvers[n]->finish_batch(batched, outcomes[n], failure)) {
-      failure.message = "picture " + std::to_string(n) + ": " + failure.message;
-      return false;
-    }
-  }
-  return true;
+  return good;
 }
 
 }  // namespace urb

@@ -25,8 +25,8 @@ struct BatchEntry {
   Plan plan;
 };
 
-// The batched part's device time (CUDA events around it on the batch's stream), the
-// iterations it made, the launches it made an iteration, and the samples and pixels of all
+// The device time from the first launch of the iterations but the last to the end of the last
+// picture's (CUDA events), the iterations made, the launches it made an iteration, and the samples and pixels of all
 // pictures.
 struct BatchTiming {
   double milliseconds = 0.0;

@@ -1232,10 +1232,20 @@ bool Solver::run(std::uint64_t first, const Observer& observer, Outcome& out, Fa
   return m.check(failure, "the result");
 }
 
-bool Solver::begin_batch(const Plan& plan, Failure& failure) {
+bool Solver::walks() const { return impl_->walk_keeps(); }
+
+cudaError_t Solver::walk(std::uint64_t done) {
+  Impl& m = *impl_;
+  if (done > 0) m.primal(false);
+  for (std::uint64_t n = 1; n < done && m.error == cudaSuccess; ++n) m.fused();
+  if (done > 0) m.dual(false);
+  return m.error;
+}
+
+bool Solver::begin_batch(const Plan& plan, Failure& failure, bool walking) {
   Impl& m = *impl_;
   m.plan = plan;
-  m.setup(plan.tgv, false);
+  m.setup(plan.tgv, walking);
   m.set_factors(plan);
   m.start(nullptr, true);
   bytes_ = m.bytes;
