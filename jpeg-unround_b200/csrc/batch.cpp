@@ -176,9 +176,9 @@ int tune_dual(const DualClass& dual, const DualBatchImage* images_device, cudaSt
 }
 
 // Pictures of kWalkSamples samples or more that the walk takes iterate by launches of their own,
-// kLanes of them at a time on streams of their own, beside the batched launches of the others: a
-// walk moves 73 bytes a sample where the two batched steps move 85, and a picture's last iteration
-// and result come while the next ones iterate. A picture's share of an iteration, batched (12 alike)
+// kLanes of them at a time, beside the batched launches of the others: a walk moves 73 bytes a sample
+// where the two batched steps move 85, and a picture's last iteration and result come while others
+// iterate. A picture's share of an iteration, batched (12 alike)
 // and by walks in three lanes: TGV grey 384^2 3.60 and 3.27 us, 512^2 6.07 and 4.49, 1024^2 19.6
 // and 16.3; TGV 4:2:0 256^2 5.12 and 3.65, 512^2 15.0 and 13.2, 1024^2 51.3 and 47.7; TV 4:2:0
 // 256^2 3.02 and 2.59, 512^2 8.29 and 6.81, 1024^2 28.7 and 24.7. Below, the host's 2.3 us a launch
@@ -192,24 +192,26 @@ bool wants_walk(const BatchEntry& e) {
   return (e.plan.tgv || f.channels() > 1) && f.channels() * f.rows * f.columns >= kWalkSamples;
 }
 
-// The pictures that walk: a stream and the event of its iterations' end each.
+// The lanes' streams, and the event of each walking picture's iterations' end.
 struct Walkers {
   std::vector<std::size_t> pictures;
-  std::vector<cudaStream_t> streams;  // of every picture of the batch; null for one without
-  std::vector<cudaEvent_t> ends;
+  std::vector<cudaEvent_t> ends;  // of every picture of the batch; null for one that does not walk
+  cudaStream_t lanes[kLanes] = {};
   cudaError_t error = cudaSuccess;
-  explicit Walkers(const std::vector<BatchEntry>& entries) {
-    streams.resize(entries.size(), nullptr);
-    ends.resize(entries.size(), nullptr);
-    for (std::size_t n = 0; n < entries.size(); ++n) {
-      if (!wants_walk(entries[n])) continue;
-      if (error == cudaSuccess) error = cudaStreamCreateWithFlags(&streams[n], cudaStreamNonBlocking);
+  void prepare(std::size_t count) {
+    ends.resize(count, nullptr);
+    for (std::size_t n : pictures) {
       if (error == cudaSuccess) error = cudaEventCreate(&ends[n]);
+    }
+    for (std::size_t k = 0; k < std::min(kLanes, pictures.size()); ++k) {
+      if (error == cudaSuccess) error = cudaStreamCreateWithFlags(&lanes[k], cudaStreamNonBlocking);
     }
   }
   ~Walkers() {
-    for (cudaStream_t s : streams) {
-      if (s != nullptr) cudaStreamDestroy(s);
+    for (cudaStream_t s : lanes) {
+      if (s == nullptr) continue;
+      cudaStreamSynchronize(s);
+      cudaStreamDestroy(s);
     }
     for (cudaEvent_t e : ends) {
       if (e != nullptr) cudaEventDestroy(e);
@@ -250,17 +252,18 @@ bool solve_batch(const std::vector<BatchEntry>& entries, cudaStream_t stream, st
   if (!check_batch(entries, failure)) return false;
   const std::uint64_t most = entries[0].plan.iterations;
   // Each picture's solver, started.
-  Walkers walkers(entries);
+  std::vector<std::unique_ptr<Solver>> solvers;
+  Walkers walkers;  // their launches are waited for before the solvers go
+  for (std::size_t n = 0; n < entries.size(); ++n) {
+    const bool walking = wants_walk(entries[n]);
+    solvers.push_back(std::make_unique<Solver>(*entries[n].frame, stream));
+    if (!solvers.back()->begin_batch(entries[n].plan, failure, walking)) return false;
+    if (walking && solvers.back()->walks()) walkers.pictures.push_back(n);
+  }
+  walkers.prepare(entries.size());
   if (walkers.error != cudaSuccess) {
     failure = {kInternal, "the batch's streams: " + describe(walkers.error)};
     return false;
-  }
-  std::vector<std::unique_ptr<Solver>> solvers;
-  for (std::size_t n = 0; n < entries.size(); ++n) {
-    const bool walking = walkers.streams[n] != nullptr;
-    solvers.push_back(std::make_unique<Solver>(*entries[n].frame, walking ? walkers.streams[n] : stream));
-    if (!solvers.back()->begin_batch(entries[n].plan, failure, walking)) return false;
-    if (walking && solvers.back()->walks()) walkers.pictures.push_back(n);
   }
   // The tables: each picture's entry, each component's, and per class the tiles and items.
   std::vector<DualBatchImage> images(entries.size());
@@ -421,32 +424,33 @@ bool solve_batch(const std::vector<BatchEntry>& entries, cudaStream_t stream, st
   outcomes.clear();
   outcomes.resize(entries.size());
   bool good = true;
-  auto finish = [&](std::size_t n) {
-    if (!good || error != cudaSuccess || solvers[n]->finish_batch(batched, outcomes[n], failure)) return;
-    failure.message = "picture " + std::to_string(n) + ": " + failure.message;
-    good = false;
-  };
-  // The walking pictures, the largest first, so that the lanes end together: a picture's iterations
-  // follow those of the one kLanes before it, which is finished while they run; the batched ones are
-  // finished beside the last walks.
+  // The walking pictures, the largest first, so that the lanes end together; each is finished, on the
+  // batch's stream, while later ones iterate, and the batched ones beside the last walks.
   std::vector<std::size_t> order = walkers.pictures;
   std::stable_sort(order.begin(), order.end(), [&](std::size_t x, std::size_t y) {
     const Geometry &p = solvers[x]->geometry(), &q = solvers[y]->geometry();
     return p.plane * p.channels > q.plane * q.channels;
   });
-  for (std::size_t k = 0; k < order.size(); ++k) {
-    const std::size_t n = order[k];
-    if (good && error == cudaSuccess) {
-      error = cudaStreamWaitEvent(walkers.streams[n], k < kLanes ? began : walkers.ends[order[k - kLanes]], 0);
-      if (error == cudaSuccess) error = solvers[n]->walk(batched);
-      if (error == cudaSuccess) error = cudaEventRecord(walkers.ends[n], walkers.streams[n]);
+  for (std::size_t k = 0; k < order.size() && error == cudaSuccess; ++k) {
+    const cudaStream_t lane = walkers.lanes[k % kLanes];
+    if (k < kLanes) error = cudaStreamWaitEvent(lane, began, 0);
+    if (error == cudaSuccess) error = solvers[order[k]]->walk(batched, lane);
+    if (error == cudaSuccess) error = cudaEventRecord(walkers.ends[order[k]], lane);
+  }
+  auto finish = [&](std::size_t n) {
+    if (good && error == cudaSuccess && walkers.ends[n] != nullptr) {
+      error = cudaStreamWaitEvent(stream, walkers.ends[n], 0);
     }
-    if (k >= kLanes) finish(order[k - kLanes]);
-  }
+    if (!good || error != cudaSuccess || solvers[n]->finish_batch(batched, outcomes[n], failure)) return;
+    failure.message = "picture " + std::to_string(n) + ": " + failure.message;
+    good = false;
+  };
+  const std::size_t last = order.size() - std::min(order.size(), kLanes);
+  for (std::size_t k = 0; k < last; ++k) finish(order[k]);
   for (std::size_t n = 0; n < entries.size(); ++n) {
-    if (std::find(order.begin(), order.end(), n) == order.end()) finish(n);
+    if (walkers.ends[n] == nullptr) finish(n);
   }
-  for (std::size_t k = order.size() - std::min(order.size(), kLanes); k < order.size(); ++k) finish(order[k]);
+  for (std::size_t k = last; k < order.size(); ++k) finish(order[k]);
   // From the first launch to the end of the last picture's iterations.
   auto until = [&](cudaEvent_t end) {
     float milliseconds = 0.0f;

@@ -1234,11 +1234,14 @@ bool Solver::run(std::uint64_t first, const Observer& observer, Outcome& out, Fa
 
 bool Solver::walks() const { return impl_->walk_keeps(); }
 
-cudaError_t Solver::walk(std::uint64_t done) {
+cudaError_t Solver::walk(std::uint64_t done, cudaStream_t on) {
   Impl& m = *impl_;
+  const cudaStream_t own = m.stream;
+  m.stream = on;
   if (done > 0) m.primal(false);
   for (std::uint64_t n = 1; n < done && m.error == cudaSuccess; ++n) m.fused();
   if (done > 0) m.dual(false);
+  m.stream = own;
   return m.error;
 }
 

@@ -95,10 +95,10 @@ class Solver {
   // batch (the state of iteration `done` current), the rest as solve() makes it: the remaining
   // iterations, the records and the result. The batch's plans record at the last iteration only.
   // `walking`: the picture may iterate by launches of its own, the walk's, where walks() says so
-  // after; walk() then puts the `done` iterations on the solver's stream (not waited for).
+  // after; walk() then puts the `done` iterations on the stream `on` (not waited for).
   bool begin_batch(const Plan& plan, Failure& failure, bool walking = false);
   bool walks() const;
-  cudaError_t walk(std::uint64_t done);
+  cudaError_t walk(std::uint64_t done, cudaStream_t on);
   bool batch_entries(DualBatchImage& image, std::vector<PrimalBatchComponent>& components);
   bool finish_batch(std::uint64_t done, Outcome& out, Failure& failure);
 
