@@ -1244,6 +1244,9 @@ template <int CR, int CC>
 __global__ void __launch_bounds__(256) conjugate_kernel(const __grid_constant__ ConjugatePair Q) {
   __shared__ double tile[kWarps][4][72];
   const ConjugateParams& P = Q.part[blockIdx.z];
+  // The conjugates of the other channels may run beside (launch_conjugate): of small pictures each
+  // launch leaves most of the device idle. What these read was whole before the first of them began.
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   constexpr int BH = 8 * CR, BW = 8 * CC;
   const int lane = threadIdx.x, b = lane >> 3, m = lane & 7;
   const int rows = P.g.rows, columns = P.g.columns, pitch = P.g.pitch;
@@ -1319,6 +1322,7 @@ __global__ void __launch_bounds__(256) conjugate_kernel(const __grid_constant__ 
     }
   }
   cta_sum(counted ? total : 0.0, P.partials);
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // done only when the launch before is
 }
 
 __global__ void __launch_bounds__(256) residual_kernel(const ResidualParams P) {
@@ -1431,13 +1435,20 @@ struct CanvasLaunch {
 
 template <int CR, int CC>
 struct ConjugateLaunch {
-  static cudaError_t run(const ConjugatePair& q, int count, cudaStream_t s) {
+  static cudaError_t run(const ConjugatePair& q, int count, bool beside, cudaStream_t s) {
     const ConjugateParams& p = q.part[0];
     const int warps = conjugate_warps(p.g, p.component);
-    dim3 grid = conjugate_grid(p.g, p.component, warps);
-    grid.z = count;
-    conjugate_kernel<CR, CC><<<grid, dim3(32, warps), 0, s>>>(q);
-    return cudaGetLastError();
+    cudaLaunchConfig_t config = {};
+    config.gridDim = conjugate_grid(p.g, p.component, warps);
+    config.gridDim.z = count;
+    config.blockDim = dim3(32, warps);
+    config.stream = s;
+    cudaLaunchAttribute early;
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    config.attrs = &early;
+    config.numAttrs = beside ? 1 : 0;
+    return cudaLaunchKernelEx(&config, conjugate_kernel<CR, CC>, q);
   }
 };
 
@@ -1669,10 +1680,11 @@ cudaError_t launch_norms(const NormParams& p, bool tgv, bool coupled, cudaStream
   return tgv ? norms_channels<true>(p, coupled, stream) : norms_channels<false>(p, coupled, stream);
 }
 
-cudaError_t launch_conjugate(const ConjugateParams* parts, int count, cudaStream_t stream) {
+cudaError_t launch_conjugate(const ConjugateParams* parts, int count, bool beside, cudaStream_t stream) {
   if (count < 1 || count > 2) return cudaErrorInvalidValue;
   const ConjugatePair pair{{parts[0], parts[count - 1]}};
-  return by_cells<ConjugateLaunch>(parts[0].component.cell_rows, parts[0].component.cell_columns, pair, count, stream);
+  return by_cells<ConjugateLaunch>(parts[0].component.cell_rows, parts[0].component.cell_columns, pair, count, beside,
+                                   stream);
 }
 
 cudaError_t launch_reductions(const Reductions& r, cudaStream_t stream) {

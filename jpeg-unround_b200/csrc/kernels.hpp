@@ -340,7 +340,9 @@ cudaError_t launch_norms(const NormParams& p, bool tgv, bool coupled, cudaStream
 struct ConjugatePair {
   ConjugateParams part[2];
 };
-cudaError_t launch_conjugate(const ConjugateParams* parts, int count, cudaStream_t stream);
+// `beside`: it may run beside the launch before it on the stream, which is one of these and not beside
+// another itself (a record of 768x512 4:2:0, Y and then Cb and Cr: 98 -> 90 us).
+cudaError_t launch_conjugate(const ConjugateParams* parts, int count, bool beside, cudaStream_t stream);
 cudaError_t launch_residual(const ResidualParams& p, cudaStream_t stream);
 // The dual step as a TMA-fed sweep (sweep.cu): `state` maps the input state's planes (fields x,
 // p1, p2 and for TGV w1, w2, r11, r22, r12, each channel after channel, one allocation), `tilde`

@@ -734,7 +734,7 @@ struct Solver::Impl {
   // With `pair`, those of channel c + 1 too (of the same cells; q1 and q2 of it `step` floats on),
   // behind c's: the count of each is returned.
   int conjugate_into(std::size_t c, const float* q1, const float* q2, double scale, const double* most_at, double* out,
-                     bool pair = false, std::size_t step = 0) {
+                     bool pair = false, std::size_t step = 0, bool beside = false) {
     if (samples != nullptr) {
       SamplesConjugateParams sp;
       sp.g = g;
@@ -767,7 +767,7 @@ struct Solver::Impl {
       cp.free = frame.components[c + k].free ? 1 : 0;
       cp.partials = out;
     }
-    if (error == cudaSuccess) error = launch_conjugate(parts, pair ? 2 : 1, stream);
+    if (error == cudaSuccess) error = launch_conjugate(parts, pair ? 2 : 1, beside, stream);
     return conjugate_count(c);
   }
 
@@ -886,11 +886,13 @@ struct Solver::Impl {
     second.out = record_sums + kMaxReductions;
     double* region = record_partials;
     const double* most_at = tgv ? record_sums + made.most : nullptr;
+    bool beside = false;  // every second launch beside the first
     for (std::size_t c = 0; c < data_channels(); ++c) {
       const float* q1 = tgv ? div2 + 2 * c * g.plane : tilde.p1 + c * g.plane;
       const float* q2 = tgv ? div2 + (2 * c + 1) * g.plane : tilde.p2 + c * g.plane;
       const bool pair = conjugate_pair(c);
-      const int n = conjugate_into(c, q1, q2, 1.0, most_at, region, pair, (tgv ? 2 : 1) * g.plane);
+      const int n = conjugate_into(c, q1, q2, 1.0, most_at, region, pair, (tgv ? 2 : 1) * g.plane, beside);
+      beside = !beside;
       for (int k = 0; k < (pair ? 2 : 1); ++k, region += n) made.dual.push_back(second.add(region, n));
       if (pair) ++c;
     }
