@@ -12,6 +12,8 @@
 #include <mutex>
 #include <thread>
 
+#include <pthread.h>
+
 namespace urb {
 
 namespace {
@@ -34,8 +36,17 @@ struct Blocks {
   std::uint64_t returned = 0;
 };
 
+Blocks& blocks();
+
+// Around a fork the list is held, so that the child, which has the forking thread alone, finds it whole
+// and free: it gives back the blocks of the arrays that it inherited.
+Blocks* make_blocks() {
+  pthread_atfork([] { blocks().lock.lock(); }, [] { blocks().lock.unlock(); }, [] { blocks().lock.unlock(); });
+  return new Blocks;
+}
+
 Blocks& blocks() {
-  static Blocks* made = new Blocks;  // never destroyed: blocks may be returned during exit
+  static Blocks* made = make_blocks();  // never destroyed: blocks may be returned during exit
   return *made;
 }
 
