@@ -53,6 +53,7 @@ Blocks& blocks() {
 }  // namespace
 
 void* reused_block(std::size_t bytes) {
+  if (bytes > std::numeric_limits<std::size_t>::max() / 4) throw std::bad_alloc();  // no sum below overflows
   Blocks& b = blocks();
   {
     std::lock_guard<std::mutex> hold(b.lock);

@@ -62,3 +62,9 @@ def test_children_made_while_blocks_are_taken():
         for thread in threads:
             thread.join()
     assert hung == 0
+
+
+def test_a_size_that_cannot_be_had_gives_none():
+    library = native._library()
+    assert not library.unround_b200_host_block(2**64 - 1)
+    assert not library.unround_b200_host_block(2**64 - 64)
