@@ -89,6 +89,8 @@ unround_status unround_b200_solve_batch(uint64_t count, const unround_input* inp
  * kept every `checkpoint_every` iterations. Every pointer is device memory of the current
  * device; the caller allocates `checkpoint_floats` floats for the checkpoints and
  * `workspace_floats` for the workspace; the work runs on `stream` and is not waited for.
+ * alpha0 and alpha1 are taken as they are: where one is negative, what lies beyond its square is
+ * scaled by alpha / |q| and what lies within by 1, forward and backward.
  * The problem's constants (made by the host model, unround_b200_model): */
 typedef struct unround_b200_unrolled {
   uint64_t images, rows, columns; /* canvases of whole 8x8 blocks */

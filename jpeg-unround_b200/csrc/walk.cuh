@@ -127,11 +127,16 @@ __device__ __forceinline__ Pair fma2(Pair a, Pair b, Pair c) {
 // packed operations against two square roots and two divisions. Their one exception, a divisor
 // whose significand is all ones, and squares and radii far from 1 (`usual` false), where an
 // intermediate could leave the range, take sqrtf and the division. Equal to those on every float
-// of six octaves above the radius, for each of 600 radii.
+// of six octaves above the radius, for each of 600 radii (tests/ball_check.cu).
+// Radii that are not usual have no `inside` (their square rounds coarsely, or to 0 or infinity): the
+// norm decides. A negative one, which only the unrolled solve takes, projects beyond its square and
+// leaves what lies within, as the adjoint has it.
 struct Ball {
   float radius, inside;
   bool usual;
-  __device__ explicit Ball(float r) : radius(r), inside(r * r * 0.999999f), usual(r > 1e-12f && r < 1e12f) {}
+  __device__ explicit Ball(float r) : radius(r), usual(r > 1e-12f && r < 1e12f) {
+    inside = usual ? r * r * 0.999999f : r < 0.0f ? r * r : -1.0f;
+  }
 };
 
 __device__ __forceinline__ float ball(float square, const Ball& B) {
