@@ -89,6 +89,8 @@ unround_status unround_b200_solve_batch(uint64_t count, const unround_input* inp
  * kept every `checkpoint_every` iterations. Every pointer is device memory of the current
  * device; the caller allocates `checkpoint_floats` floats for the checkpoints and
  * `workspace_floats` for the workspace; the work runs on `stream` and is not waited for.
+ * A bounded wait of a kernel that runs out (a device at fault) leaves a NaN in the output of a
+ * forward pass, and in the gradient of sigma of a backward pass: nothing waits here to return it.
  * alpha0 and alpha1 are taken as they are: where one is negative, what lies beyond its square is
  * scaled by alpha / |q| and what lies within by 1, forward and backward.
  * The problem's constants (made by the host model, unround_b200_model): */
@@ -307,9 +309,10 @@ unround_status unround_b200_result_intervals(const unround_result* result, doubl
  * device): every wait of a kernel on an mbarrier is bounded, and one that runs out sets an error
  * word that the solve reports as UNROUND_ERROR_INTERNAL ("a bounded wait of the sweep ran out")
  * after draining the loads still in flight. This sets the tries that the dual sweep's compute
- * warps give a chunk of their ring, for the solves of this process from now on: `tries` >= 0
- * sets it, a negative value puts back the full limit (2^22). It returns the limit before. With
- * 0, every sweep gives up at its first chunk although its loads complete as usual: a test of
+ * warps (a walk's warps of the dual step) give a chunk of their ring, for the solves of this
+ * process from now on: `tries` >= 0 sets it, a negative value puts back the full limit (2^22). It
+ * returns the limit before. With 0, every sweep and walk gives up at its first chunk although its
+ * loads complete as usual: a test of
  * the failure path that neither faults nor hangs the device. */
 int64_t unround_b200_set_ring_wait_limit(int64_t tries);
 

@@ -235,6 +235,21 @@ __device__ __forceinline__ void after_launch_before() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// A walk of which a wait ran out leaves a NaN in its x~ and in x of every state after (walk_unrolled.cu).
+// What a pass returns has one then too: where `from` has one, its output, or (`grads`) its picture's
+// gradient of sigma, the one to which every pixel adds.
+__global__ void __launch_bounds__(256) failed_kernel(const float4* from, std::size_t count, std::size_t picture,
+                                                     float* output, double* grads) {
+  after_launch_before();
+  const std::size_t stride = static_cast<std::size_t>(gridDim.x) * 256;
+  for (std::size_t k = static_cast<std::size_t>(blockIdx.x) * 256 + threadIdx.x; k < count; k += stride) {
+    const float4 x = from[k];
+    if (!(isnan(x.x) || isnan(x.y) || isnan(x.z) || isnan(x.w))) continue;
+    if (output != nullptr) output[4 * k] = __int_as_float(0x7fc00000);
+    if (grads != nullptr) atomicAdd(grads + 4 * k / picture, static_cast<double>(__int_as_float(0x7fc00000)));
+  }
+}
+
 // ---- Adjoint. `a` holds the adjoint of s_k (the dual step's output) and, as its ninth plane,
 // that of v of the primal step P_{k+1} after it; the kernels write the adjoint of s_{k-1} into
 // `b` and the adjoint of x~_k into `xt_bar`. Gradients: [0] alpha0, [1] alpha1, [2] tau,
@@ -649,6 +664,7 @@ cudaError_t walk(const CUtensorMap& from, const Problem& q, float* to, float* ne
                  to + 7 * q.plane};
   d.rho = q.rho;
   d.rest = 1.0f - q.rho;
+  d.ring_wait_limit = ring_wait_limit();
   w.step.next = next;
   w.images = q.images;
   w.lower = q.lower;
@@ -663,6 +679,13 @@ cudaError_t walk(const CUtensorMap& from, const Problem& q, float* to, float* ne
   w.tau = q.tau;
   w.sigma = q.sigma;
   return launch_walk_unrolled(from, w, stream);
+}
+
+cudaError_t tell_failed(const Problem& q, const float* from, float* output, double* grads, cudaStream_t stream) {
+  const std::size_t count = q.plane / 4;  // whole blocks
+  const auto ctas = static_cast<unsigned>(std::min<std::size_t>((count + 255) / 256, 1184));
+  return launch_next(failed_kernel, dim3(ctas), dim3(256), 0, stream, reinterpret_cast<const float4*>(from), count,
+                     q.plane / q.images, output, grads);
 }
 
 std::string check(const unround_b200_unrolled* u) {
@@ -785,6 +808,8 @@ extern "C" unround_status unround_b200_unrolled_forward(const unround_b200_unrol
     current = next;
     current_map = next_map;
   }
+  // x of s_{N-1} (the last walk marks the output itself).
+  if (n > 1 && error == cudaSuccess) error = urb::tell_failed(q, current, output, nullptr, on);
   if (error == cudaSuccess) error = cudaGetLastError();
   if (error != cudaSuccess) {
     urb::tell(message, message_size, std::string("the device failed in the unrolled solve: ") + cudaGetErrorString(error));
@@ -859,6 +884,11 @@ extern "C" unround_status unround_b200_unrolled_backward(const unround_b200_unro
       const std::uint64_t step = k - 1 - k0;  // s_{k-1} is storage_of(seg, step)
       float* const to = storage_of(seg, step + 1);
       error = urb::walk(step == 0 ? checkpoint_forward[seg] : recomputed_forward[step - 1], q, to, to + 8 * plane, on);
+    }
+    // The marks of these walks reach sigma's gradient through D_k's adjoint; of the last, whose x~_N nothing
+    // reads, they do here.
+    if (k1 == n && k0 + 1 < n && error == cudaSuccess) {
+      error = urb::tell_failed(q, storage_of(seg, n - 1 - k0) + 8 * plane, nullptr, grads + 3 * problem->images, on);
     }
     // Backwards through the segment: at iteration k, D_k (k < N) then P_k.
     for (std::uint64_t k = k1; k > k0; --k) {
