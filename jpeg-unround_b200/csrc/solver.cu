@@ -57,6 +57,13 @@ int samples_kernels() {
 // 1.04 -> 0.84 ms without, 512x512 2.2 -> 1.9; photographs and larger alike either way).
 constexpr std::uint64_t kGraphIterations = 8;
 
+// The samples of the walks that follow a record before it is looked at: 6 of 160x120 (3.7 us each), 6
+// of 512^2 of one channel, 1 from 768x512 of three (18 us) on.
+// TGV solves that stop at a tolerance, a record every 100 iterations, with all of them up to the next
+// record in front of the look and now: 512^2 of one channel 3.48 -> 2.85 ms, 768x512 4:2:0 13.0 -> 11.4,
+// 2048^2 4:2:0 158.7 -> 141.5, 4032x3024 4:2:0 482.5 -> 431.8; a record every 10 of the last 478 -> 476.
+constexpr std::uint64_t kLeadSamples = std::uint64_t{1} << 21;
+
 bool group_graphs() {
   const char* value = std::getenv("UNROUND_B200_GRAPHS");
   return value == nullptr || std::strcmp(value, "0") != 0;
@@ -923,6 +930,15 @@ struct Solver::Impl {
     if (error == cudaSuccess) error = cudaEventRecord(record_done, stream);
   }
 
+  // Whether the record on the stream is done.
+  bool record_there() {
+    if (error != cudaSuccess) return true;
+    const cudaError_t there = cudaEventQuery(record_done);
+    if (there == cudaErrorNotReady) return false;
+    if (error == cudaSuccess) error = there;
+    return true;
+  }
+
   Record collect_record() {
     Record r;
     r.iteration = made.iteration;
@@ -1169,9 +1185,12 @@ bool Solver::run(std::uint64_t first, const Observer& observer, Outcome& out, Fa
     return false;
   };
   auto recorded = [&](std::uint64_t n) { return (every > 0 && n % every == 0) || n == most; };
-  // With the walk, the iterations after a record that keep nothing follow it on the stream before it
-  // is looked at: they leave alone what the result is made from (zeta and v of the last kept primal
-  // step). Everything else settles it at once.
+  // With the walk, iterations after a record that keep nothing follow it on the stream before it is
+  // looked at: they leave alone what the result is made from (zeta and v of the last kept primal
+  // step). Everything else settles it at once. No more follow than cover the host's look (about 15 us,
+  // when the record is done): where the solve stops at it they are work for nothing.
+  const std::uint64_t lead =
+      std::clamp<std::uint64_t>(kLeadSamples / std::max<std::uint64_t>(static_cast<std::uint64_t>(samples), 1), 1, 6);
   auto take = [&](std::uint64_t iteration) -> bool {
     m.enqueue_record(iteration);
     pending = true;
@@ -1189,7 +1208,8 @@ bool Solver::run(std::uint64_t first, const Observer& observer, Outcome& out, Fa
   if (!stopped && first < most) m.primal(recorded(first + 1));
   while (!stopped && iteration < most && m.error == cudaSuccess) {
     const std::uint64_t next = iteration + 1;
-    if (pending && (recorded(next) || recorded(next + 1)) && settle()) {
+    if (pending && (recorded(next) || recorded(next + 1) || iteration >= m.made.iteration + lead || m.record_there()) &&
+        settle()) {
       stopped = true;
       iteration = m.made.iteration;
       break;
