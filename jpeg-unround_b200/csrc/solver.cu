@@ -179,15 +179,19 @@ struct Solver::Impl {
 
   // A state's fields in one allocation, each field's channels one after another, in the order
   // x, p1, p2, w1, w2, r11, r22, r12: the planes of the sweep's TMA box (sweep.cu).
-  // With `tilde`, x~'s planes lie behind them (the walk's box, walk.cuh).
-  Fields fields(bool with_tgv, float** tilde = nullptr) {
+  // With `tilde`, x~'s planes lie behind them (the walk's box, walk.cuh). Without `with_x`, no x.
+  Fields fields(bool with_tgv, float** tilde = nullptr, bool with_x = true) {
     const std::size_t n = g.plane * g.channels;
     const int count = with_tgv ? 8 : 3;
-    float* block = allocate<float>(n * (count + (tilde != nullptr ? 1 : 0)));
+    float* block = allocate<float>(n * (count + (tilde != nullptr ? 1 : 0) - (with_x ? 0 : 1)));
     if (tilde != nullptr) *tilde = block != nullptr ? block + n * count : nullptr;
     Fields f;
     if (block == nullptr) return f;
-    f.x = block;
+    if (with_x) {
+      f.x = block;
+    } else {
+      block -= n;
+    }
     f.p1 = block + n;
     f.p2 = block + 2 * n;
     if (with_tgv) {
@@ -285,7 +289,9 @@ struct Solver::Impl {
     walks = ((whole && kernels == Kernels::walk) || (swept_samples && samples_layout == 3 && large)) && walk_takes(g);
     fusable = walks || (swept_samples && samples_layout != 3) || (whole && kernels == Kernels::fused);
     for (int s = 0; s < 2; ++s) state[s] = fields(with_tgv, walks ? &xts[s] : nullptr);
-    tilde = fields(with_tgv);
+    // x of the tilde point is x~ itself. (With a plane for it and the walk's second x~, a picture that
+    // filled the device before the walk did not fit any more.)
+    tilde = fields(with_tgv, nullptr, false);
     if (!walks) xts[0] = allocate<float>(n);
     xt = xts[0];
     xt_id = 0;
