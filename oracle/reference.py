@@ -46,6 +46,11 @@ class _Start(ctypes.Structure):
     )
 
 
+class NotBuilt(FileNotFoundError):
+    """The reference's solver is not there: it is compiled from the reference's sources, which not every
+    machine has."""
+
+
 def available() -> bool:
     return LIBRARY.is_file()
 
@@ -53,7 +58,7 @@ def available() -> bool:
 @functools.cache
 def _library() -> ctypes.CDLL:
     if not LIBRARY.is_file():
-        raise FileNotFoundError(f"{LIBRARY} is not built: run make -C oracle/ref")
+        raise NotBuilt(f"{LIBRARY} is not built: run make -C oracle/ref")
     lib = ctypes.CDLL(str(LIBRARY))
     u64p = ctypes.POINTER(ctypes.c_uint64)
     dp = ctypes.POINTER(ctypes.c_double)
