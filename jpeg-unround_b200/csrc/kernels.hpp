@@ -451,8 +451,12 @@ cudaError_t launch_iteration(const CUtensorMap& state, const CUtensorMap& tilde,
 // The same iteration as a walk (walk.cuh), which takes what iteration_takes says: the default. Its
 // map boxes two rows of `count` planes, a state's and behind them those of x~ that its primal step
 // made; `p.next` lies likewise behind p.dual.out.
-// And planes of less than 2^30 samples: offsets within one are 32 bits of bytes.
-inline bool walk_takes(const Geometry& g) { return g.plane < (std::size_t{1} << 30); }
+// And planes of less than 2^30 samples: offsets within one are 32 bits of bytes; and balls of usual radii,
+// whose squares the walk compares where the other kernels compare norms.
+constexpr bool usual_radius(float r) { return r > 1e-12f && r < 1e12f; }
+inline bool walk_takes(const Geometry& g, float radius, float radius0) {
+  return g.plane < (std::size_t{1} << 30) && usual_radius(radius) && usual_radius(radius0);
+}
 bool make_walk_map(CUtensorMap& map, const float* planes, const Geometry& g, int count);
 // What a walk keeps for a record: nothing; its primal step's zeta, v and sums of G's terms (each
 // warp's into p.partials, *partials of them a component, at most walk_partials); its dual step's

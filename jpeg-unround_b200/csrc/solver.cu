@@ -249,6 +249,9 @@ struct Solver::Impl {
     if (error == cudaSuccess) error = cudaStreamSynchronize(stream);  // the staged copies' sources
   }
 
+  // The radius of p's balls.
+  float radius() const { return static_cast<float>(tgv ? plan.alpha1 : plan.alpha); }
+
   void setup(bool with_tgv, bool solving = true) {
     tgv = with_tgv;
     const std::size_t n = g.plane * g.channels;
@@ -286,7 +289,8 @@ struct Solver::Impl {
                        iteration_takes(g, components.data(), static_cast<int>(components.size()));
     const bool swept_samples = samples != nullptr && solving && samples_layout != 0 && samples_iteration_takes(g);
     const bool large = static_cast<std::size_t>(g.channels) * g.rows * g.columns >= kSamplesWalk;
-    walks = ((whole && kernels == Kernels::walk) || (swept_samples && samples_layout == 3 && large)) && walk_takes(g);
+    walks = ((whole && kernels == Kernels::walk) || (swept_samples && samples_layout == 3 && large)) &&
+            walk_takes(g, radius(), with_tgv ? static_cast<float>(plan.alpha0) : 1.0f);
     fusable = walks || (swept_samples && samples_layout != 3) || (whole && kernels == Kernels::fused);
     for (int s = 0; s < 2; ++s) state[s] = fields(with_tgv, walks ? &xts[s] : nullptr);
     // x of the tilde point is x~ itself. (With a plane for it and the walk's second x~, a picture that
@@ -618,7 +622,7 @@ struct Solver::Impl {
     }
     dp.rho = static_cast<float>(plan.relaxation);
     dp.rest = static_cast<float>(1.0 - plan.relaxation);
-    dp.radius = static_cast<float>(tgv ? plan.alpha1 : plan.alpha);
+    dp.radius = radius();
     dp.radius0 = static_cast<float>(plan.alpha0);
     dp.error = error_word;
     dp.ring_wait_limit = ring_wait_limit();

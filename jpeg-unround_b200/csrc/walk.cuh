@@ -128,15 +128,14 @@ __device__ __forceinline__ Pair fma2(Pair a, Pair b, Pair c) {
 // whose significand is all ones, and squares and radii far from 1 (`usual` false), where an
 // intermediate could leave the range, take sqrtf and the division. Equal to those on every float
 // of six octaves above the radius, for each of 600 radii (tests/ball_check.cu).
-// Radii that are not usual have no `inside` (their square rounds coarsely, or to 0 or infinity): the
-// norm decides. A negative one, which only the unrolled solve takes, projects beyond its square and
-// leaves what lies within, as the adjoint has it.
+// A solve's radii are usual (walk_takes). The unrolled solve takes `any`: of a tiny one, whose square
+// rounds coarsely or to 0, `inside` is negative and the norm decides; a negative one projects beyond its
+// square and leaves what lies within, as the adjoint has it.
 struct Ball {
   float radius, inside;
   bool usual;
-  __device__ explicit Ball(float r) : radius(r), usual(r > 1e-12f && r < 1e12f) {
-    inside = usual ? r * r * 0.999999f : r < 0.0f ? r * r : -1.0f;
-  }
+  __device__ explicit Ball(float r, bool any = false)
+      : radius(r), inside(any ? r * r * 0.999999f - 1e-25f : r * r * 0.999999f), usual(usual_radius(r)) {}
 };
 
 __device__ __forceinline__ float ball(float square, const Ball& B) {
@@ -496,7 +495,7 @@ struct Walk {
         square_p = c == 0 ? square : add2(square_p, square);
       }
     }
-    const Ball unit(radius());
+    const Ball unit(radius(), UNROLLED);
     Pair scale = 0;
     if constexpr (COUPLED) scale = ball2(square_p, unit);
 #pragma unroll
@@ -551,7 +550,7 @@ struct Walk {
     };
     auto left_of = [&](int q, int c, Pair p) -> Pair { return pair(own_row[exchange(q, c) + before], first(p)); };
     if constexpr (TGV) {
-      const Ball unit(radius0());
+      const Ball unit(radius0(), UNROLLED);
       Pair r11[C], r22[C], r12[C];
       Pair square = 0;
 #pragma unroll
@@ -724,7 +723,7 @@ struct Walk {
       square = total;
     }
     if (mine) {
-      const float q1 = __fmul_rn(step1, ball(square, Ball(radius())));
+      const float q1 = __fmul_rn(step1, ball(square, Ball(radius(), UNROLLED)));
       float* to = shared + W::EXCHANGE + (row < kChunk - 1 ? row : row + (k & 1)) * W::ROW - 1 - (k & 1);
       to[exchange(0, c)] =
           REST_FIRST ? fmaf(P.rest, old1, __fmul_rn(P.rho, q1)) : fmaf(P.rho, q1, __fmul_rn(P.rest, old1));

@@ -9,8 +9,9 @@ __device__ float by_norm(float square, float radius) {
   return norm > radius ? radius / norm : 1.0f;
 }
 
-__global__ void check(float radius, unsigned first, unsigned stride, unsigned count, unsigned long long* wrong) {
-  const urb::Ball ball(radius);
+// `any`: of the unrolled solve, else of a solve, whose radii are usual.
+__global__ void check(float radius, bool any, unsigned first, unsigned stride, unsigned count, unsigned long long* wrong) {
+  const urb::Ball ball(radius, any);
   unsigned long long mine = 0;
   for (unsigned k = blockIdx.x * blockDim.x + threadIdx.x; k < count; k += gridDim.x * blockDim.x) {
     const float x = __uint_as_float(first + k * stride);
@@ -28,12 +29,12 @@ __global__ void check(float radius, unsigned first, unsigned stride, unsigned co
 }  // namespace
 
 // The number of them at which a scale differs, or -1 where the device failed.
-extern "C" long long ball_check(float radius, unsigned first, unsigned stride, unsigned count) {
+extern "C" long long ball_check(float radius, int any, unsigned first, unsigned stride, unsigned count) {
   unsigned long long* wrong = nullptr;
   unsigned long long host = 0;
   if (cudaMalloc(&wrong, sizeof(host)) != cudaSuccess) return -1;
   bool good = cudaMemset(wrong, 0, sizeof(host)) == cudaSuccess;
-  if (good) check<<<592, 256>>>(radius, first, stride, count, wrong);
+  if (good) check<<<592, 256>>>(radius, any != 0, first, stride, count, wrong);
   good = good && cudaMemcpy(&host, wrong, sizeof(host), cudaMemcpyDeviceToHost) == cudaSuccess;
   cudaFree(wrong);
   return good ? static_cast<long long>(host) : -1;
