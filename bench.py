@@ -797,15 +797,17 @@ def _large_arm(args: argparse.Namespace, rank: int, world: int) -> None:
 
 
 def _unrolled_forward_launches(iterations: int) -> int:
-    """The start, the first primal step, and N - 1 walks (a dual step and the next primal step each)."""
-    return iterations + 1
+    """The start, the first primal step, N - 1 walks (a dual step and the next primal step each), and the
+    look for one that failed."""
+    return iterations + 1 + (iterations > 1)
 
 
 def _unrolled_backward_launches(iterations: int, every: int) -> int:
     """Per segment of checkpoints K apart the walks that recompute its states, then the dual steps'
-    adjoints (N - 1) and the primal steps' adjoints (N)."""
-    launches = sum(min(k0 + every, iterations) - k0 - 1 for k0 in range(0, iterations, every))
-    return launches + (iterations - 1) + iterations
+    adjoints (N - 1) and the primal steps' adjoints (N); and the look for a failed walk where the last
+    segment has one."""
+    walks = [min(k0 + every, iterations) - k0 - 1 for k0 in range(0, iterations, every)]
+    return sum(walks) + (walks[-1] > 0) + (iterations - 1) + iterations
 
 
 def _unrolled_measure(steps: int, warmup: int, rank: int) -> dict:

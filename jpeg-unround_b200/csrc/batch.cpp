@@ -177,13 +177,15 @@ int tune_dual(const DualClass& dual, const DualBatchImage* images_device, cudaSt
 
 // Pictures of kWalkSamples samples or more that the walk takes iterate by launches of their own,
 // kLanes of them at a time, beside the batched launches of the others: a walk moves 73 bytes a sample
-// where the two batched steps move 85, and a picture's last iteration and result come while others
-// iterate. A picture's share of an iteration, batched (12 alike)
-// and by walks in three lanes: TGV grey 384^2 3.60 and 3.27 us, 512^2 6.07 and 4.49, 1024^2 19.6
+// where the two batched steps move 85, and where nothing is batched a picture's last iteration and
+// result come while others iterate. A picture's share of an iteration, batched (12 alike) and by walks in
+// three lanes: TGV grey 384^2 3.60 and 3.27 us, 512^2 6.07 and 4.49, 1024^2 19.6
 // and 16.3; TGV 4:2:0 256^2 5.12 and 3.65, 512^2 15.0 and 13.2, 1024^2 51.3 and 47.7; TV 4:2:0
 // 256^2 3.02 and 2.59, 512^2 8.29 and 6.81, 1024^2 28.7 and 24.7. Below, the host's 2.3 us a launch
 // is what many small pictures would wait for (TV 4:2:0 192^2 2.39 and 2.55, 128^2 1.73 batched). TV
-// of one channel stays batched: its batched sweep fuses another product of a sum than the walk does.
+// of one channel stays batched: its batched sweep fuses another product of a sum than the walk does. (That
+// makes a mix with many of them slower than one picture after another, which walk: 64 pictures 42,029
+// against 44,658 Mpx*iter/s.)
 constexpr std::size_t kWalkSamples = 1 << 17;
 constexpr std::size_t kLanes = 3;
 
@@ -424,8 +426,9 @@ bool solve_batch(const std::vector<BatchEntry>& entries, cudaStream_t stream, st
   outcomes.clear();
   outcomes.resize(entries.size());
   bool good = true;
-  // The walking pictures, the largest first, so that the lanes end together; each is finished, on the
-  // batch's stream, while later ones iterate, and the batched ones beside the last walks.
+  // The walking pictures, the largest first, so that the lanes end together. Each is finished on the
+  // batch's stream, behind the batched iterations, and where there are none while later ones iterate; the
+  // batched ones beside the last walks.
   std::vector<std::size_t> order = walkers.pictures;
   std::stable_sort(order.begin(), order.end(), [&](std::size_t x, std::size_t y) {
     const Geometry &p = solvers[x]->geometry(), &q = solvers[y]->geometry();

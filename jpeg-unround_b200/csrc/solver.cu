@@ -36,8 +36,8 @@ Kernels chosen_kernels() {
 // kSamplesWalk samples on); 0 two launches (the dual sweep, then the primal kernel:
 // UNROUND_B200_KERNELS=split, and what the walk does not take); 1 the fused sweep of iteration.cu
 // (=fused); 2 the dual sweep with the primal step in it (=sweep). Smaller pictures than kSamplesWalk
-// keep the two launches that measure_samples tells of them (64x64 of three channels: 13-21 us an
-// iteration; the walk, of 128x128, takes 4.5).
+// keep the two launches that measure_samples is known to tell of them, not for their speed (64x64 of
+// three channels: 13-21 us an iteration; the walk, of 128x128, takes 4.5).
 constexpr std::size_t kSamplesWalk = 1 << 15;
 
 int samples_kernels() {

@@ -27,18 +27,23 @@
 // (dual_strip of sweep.cu, primal_block_row of kernels.cu; which product of a sum is fused is
 // written out), so the iterates are theirs bit for bit. Every wait is bounded: one that runs out
 // sets the error word, the other warps see it and leave, and the copies in flight are waited for.
+// On every path a slot that a copy went to is waited for before its barrier is armed again and before
+// the CTA leaves: a chunk's slots by the warps that read them, before they arrive at `drained`, which
+// the copying warp waits for before it fills one again or leaves; slot 0, of which strips at the top
+// read nothing, by warp 0; after a wait that ran out, all that are on their way by the copying warp. (No
+// warp waited for slot 0 at first: its barrier could be armed in an unfinished phase, or a copy land in
+// the shared memory of a CTA that had left. Four solves on four streams reported a failed launch.)
 //
 // What bounds it: instructions, not memory. A chunk of three channels takes 3,900
-// warp-instructions (5.1 a sample; the two launches take 10.5) over 8 warps, two CTAs an SM by
+// warp-instructions (5.4 a sample with a strip's start; the two launches take 10.5) over 8 warps, two CTAs an SM by
 // shared memory; they issue at 1.7 an SM and cycle, held by the latency of dependent operations and
 // by instruction fetch, so that code size counts (the edges' tests are folded into addresses, and
 // what is rarely run is not inlined: 4032x3024 TV 331 -> 261 us). Its rows are there when a chunk
 // begins: of 56 looks at the ring, 55 need no wait. A launch's CTAs start on the places that the one
 // before leaves (programmatic dependent launch) and wait for its end with their barriers and
 // factors ready: 1-5 us of an iteration (160x120 5.2 -> 3.7, 2048^2 of three channels 174 -> 168).
-// They let the next launch's in only after their own wait. Let in at once, launches waited in chains,
-// as deep as small grids leave places, and with four solves on streams of their own the device
-// reported a failed launch.
+// They let the next launch's in only after their own wait, so that one launch waits at a time: let in at
+// once, launches wait in chains, as deep as small grids leave places, and hold those of other solves.
 // Measured, an iteration before (two or three launches, in graphs of eight) and after: TV grey
 // 160x120 12.6 -> 3.7 us, 512^2 13.3 -> 4.5; TGV grey 512^2 18.4 -> 8.4, 2048^2 74 -> 64; TGV 4:2:0
 // 768x512 36.7 -> 18.2, 2048^2 200 -> 167; TV 4:2:0 1919x1083 63.2 -> 43.9, 2048^2 101 (two CTAs an
