@@ -133,14 +133,18 @@ __device__ __forceinline__ Pair fma2(Pair a, Pair b, Pair c) {
 // whose significand is all ones, and squares and radii far from 1 (`usual` false), where an
 // intermediate could leave the range, take sqrtf and the division. Equal to those on every float
 // of six octaves above the radius, for each of 600 radii (tests/ball_check.cu).
-// A solve's radii are usual (walk_takes). The unrolled solve takes `any`: of a tiny one, whose square
+// A solve's radii are usual (walk_takes). The unrolled solve takes any(): of a tiny one, whose square
 // rounds coarsely or to 0, `inside` is negative and the norm decides; a negative one projects beyond its
 // square and leaves what lies within, as the adjoint has it.
 struct Ball {
   float radius, inside;
   bool usual;
-  __device__ explicit Ball(float r, bool any = false)
-      : radius(r), inside(any ? r * r * 0.999999f - 1e-25f : r * r * 0.999999f), usual(usual_radius(r)) {}
+  __device__ explicit Ball(float r) : radius(r), inside(r * r * 0.999999f), usual(r > 1e-12f && r < 1e12f) {}
+  static __device__ __forceinline__ Ball any(float r) {
+    Ball ball(r);
+    ball.inside = r * r * 0.999999f - 1e-25f;
+    return ball;
+  }
 };
 
 __device__ __forceinline__ float ball(float square, const Ball& B) {
@@ -416,6 +420,13 @@ struct Walk {
   __device__ __forceinline__ float sigma(int c) const { return UNROLLED ? image_sigma : Q.dual.sigma[c]; }
   __device__ __forceinline__ float radius() const { return UNROLLED ? image_alpha1 : Q.dual.radius; }
   __device__ __forceinline__ float radius0() const { return UNROLLED ? image_alpha0 : Q.dual.radius0; }
+  static __device__ __forceinline__ Ball ball_of(float r) {
+    if constexpr (UNROLLED) {
+      return Ball::any(r);
+    } else {
+      return Ball(r);
+    }
+  }
   // Row i of the picture among the rows of a plane; an offset within a plane in bytes.
   using Offset = std::conditional_t<UNROLLED, std::size_t, unsigned>;
   __device__ __forceinline__ Offset plane_row(int i) const {
@@ -500,7 +511,7 @@ struct Walk {
         square_p = c == 0 ? square : add2(square_p, square);
       }
     }
-    const Ball unit(radius(), UNROLLED);
+    const Ball unit = ball_of(radius());
     Pair scale = 0;
     if constexpr (COUPLED) scale = ball2(square_p, unit);
 #pragma unroll
@@ -555,7 +566,7 @@ struct Walk {
     };
     auto left_of = [&](int q, int c, Pair p) -> Pair { return pair(own_row[exchange(q, c) + before], first(p)); };
     if constexpr (TGV) {
-      const Ball unit(radius0(), UNROLLED);
+      const Ball unit = ball_of(radius0());
       Pair r11[C], r22[C], r12[C];
       Pair square = 0;
 #pragma unroll
@@ -728,7 +739,7 @@ struct Walk {
       square = total;
     }
     if (mine) {
-      const float q1 = __fmul_rn(step1, ball(square, Ball(radius(), UNROLLED)));
+      const float q1 = __fmul_rn(step1, ball(square, ball_of(radius())));
       float* to = shared + W::EXCHANGE + (row < kChunk - 1 ? row : row + (k & 1)) * W::ROW - 1 - (k & 1);
       to[exchange(0, c)] =
           REST_FIRST ? fmaf(P.rest, old1, __fmul_rn(P.rho, q1)) : fmaf(P.rho, q1, __fmul_rn(P.rest, old1));

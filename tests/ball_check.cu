@@ -11,7 +11,7 @@ __device__ float by_norm(float square, float radius) {
 
 // `any`: of the unrolled solve, else of a solve, whose radii are usual.
 __global__ void check(float radius, bool any, unsigned first, unsigned stride, unsigned count, unsigned long long* wrong) {
-  const urb::Ball ball(radius, any);
+  const urb::Ball ball = any ? urb::Ball::any(radius) : urb::Ball(radius);
   unsigned long long mine = 0;
   for (unsigned k = blockIdx.x * blockDim.x + threadIdx.x; k < count; k += gridDim.x * blockDim.x) {
     const float x = __uint_as_float(first + k * stride);
